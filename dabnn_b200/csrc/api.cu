@@ -60,6 +60,32 @@ bool make_f32_tensor_map(CUtensorMap_st* map, float* base, int rank, const unsig
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+typedef CUresult (*TensorMapEncodeIm2col)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const int*,
+                                          const int*, cuuint32_t, cuuint32_t, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                          CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+bool make_f32_im2col_map(CUtensorMap_st* map, const float* base, int n, int h, int w, int c, int kh, int kw, int pad_h, int pad_w, int stride_h,
+                         int stride_w, int dil_h, int dil_w, int channels, int pixels) {
+    static const TensorMapEncodeIm2col encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult st;
+        cudaFree(nullptr);
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeIm2col", &fn, 12000, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<TensorMapEncodeIm2col>(fn);
+    }();
+    if (!encode || !base) return false;
+    const cuuint64_t row = (cuuint64_t)c * 4;
+    const cuuint64_t d[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n}, s[3] = {row, row * w, row * w * h};
+    const int lower[2] = {-pad_w, -pad_h}, upper[2] = {pad_w - (kw - 1) * dil_w, pad_h - (kh - 1) * dil_h};   // of the window's first tap
+    const cuuint32_t e[4] = {1, (cuuint32_t)stride_w, (cuuint32_t)stride_h, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), d, s, lower, upper, (cuuint32_t)channels, (cuuint32_t)pixels, e,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool make_u8_tensor_map(CUtensorMap_st* map, const unsigned char* base, int rank, const unsigned long long* dims,
                         const unsigned long long* strides_bytes, const unsigned* box) {
     const TensorMapEncode encode = tensor_map_encoder();

@@ -1,14 +1,27 @@
-// 1x1 float convolution (a plain GEMM: pixels x Cin times Cin x Cout) on tcgen05.mma kind::tf32 with fp32-grade
-// accuracy (3xTF32), fed by TMA: no thread gathers an operand.
+// Float convolution as a TMA-fed GEMM (pixels x taps * Cin times taps * Cin x Cout) on tcgen05.mma kind::tf32 with
+// fp32-grade accuracy (3xTF32): no thread gathers an operand.
 //
-// The tensor core truncates its fp32 operands to tf32, so the raw fp32 tile that a tiled TMA load drops into shared
-// memory (128 rows x 32 floats, 128-byte-swizzled: exactly the K-major layout the MMA reads) IS the head x_hi of the
-// split x = x_hi + x_lo.  Four converter warps compute the remainders x_lo = x - trunc(x) into a second tile of the same
-// layout (same offsets, so the swizzle never has to be undone), for the pixel tile and for the weight tile alike, and
-// the MMA warp issues hi*W_hi + hi*W_lo + lo*W_hi per 8-float slice into a TMEM accumulator.
+// K runs over (window tap, 32-channel group).  A stage's pixel tile - 128 consecutive output pixels, 32 floats each - is
+// one TMA load: for 1x1 / stride 1 a box of the [pixels][Cin] matrix, otherwise an im2col-mode load, in which the copy
+// engine itself walks the window positions of 128 output pixels (row and image ends, stride, dilation, zero fill for
+// padding), so a tile has no waste at row ends and every Cin % 4 == 0 window costs the same as a 1x1.  Channels beyond
+// Cin read as zeros in both operands.
+//
+// The tensor core truncates its fp32 operands to tf32, so the raw fp32 tile that a load drops into shared memory
+// (128 rows x 32 floats, 128-byte-swizzled: exactly the K-major layout the MMA reads) IS the head x_hi of the split
+// x = x_hi + x_lo.  Eight converter warps compute the remainders x_lo = x - trunc(x) into a second tile of the same
+// layout (same offsets, so the swizzle never has to be undone), for the pixel tile and for the weight tile alike.  The
+// weight remainders follow the weights directly, so per 8-float slice the MMA warp issues hi * [W_hi; W_lo] as one
+// instruction of twice the width - the pixel operand is read once for both - and lo * W_hi, into two halves of a TMEM
+// accumulator that the epilogue adds.
+//
+// What bounds it: the shared-memory pipe.  Per 128 x 128 x 32 stage the MMAs read 80 KB, the converters move 64 KB and
+// the loads write 32 KB - about 1400 cycles at 128 B per cycle - for 864 cycles of tensor math.  A 3x3 convolution of 64
+// images of 28x28x128 to 128 channels takes 81 us here (182 TFLOP/s of fp32 products, of 340 at the tf32 issue peak); on
+// the mma.sync kernel, whose threads gather the windows, it took 364 us.
 //
 // One persistent CTA per SM walks (pixel tile, channel block) pairs, channel blocks innermost so that a pixel tile
-// is fetched from HBM once and re-read from L2.  Warps: 0 TMA loads, 1 - 4 converters, 5 MMA issue, 6 - 21 epilogue
+// is fetched from HBM once and re-read from L2.  Warps: 0 TMA loads, 1 - 8 converters, 9 MMA issue, 10 - 25 epilogue
 // (tcgen05.ld, bias, affine, relu, 128-byte-swizzled staging boxes, TMA tensor stores).  Every wait is bounded; a wait
 // that gives up records a code (41 loader, 42 converters, 43 / 44 MMA thread waiting for an accumulator / a stage,
 // 45 epilogue), raises the CTA's abort flag, and the CTA frees its tensor memory and returns.
@@ -17,13 +30,19 @@
 
 namespace dabnn {
 
-constexpr int FG_N = 128;                      // largest channel block (the accumulators lie FG_N columns apart)
+constexpr int FG_N = 128;                      // largest channel block; an accumulator has two halves of that many columns
 constexpr int FG_CHUNK = 32;                   // floats of K per stage: one 128-byte row
-constexpr int FG_CONVERTERS = 128, FG_EPILOGUE = 512;
+constexpr int FG_CONVERTERS = 256, FG_EPILOGUE = 512;
 constexpr int FG_THREADS = 32 + FG_CONVERTERS + 32 + FG_EPILOGUE;
 constexpr int FG_MMA_WARP = 1 + FG_CONVERTERS / 32;
 constexpr int FG_EPI_WARP0 = FG_MMA_WARP + 1;
-constexpr int FG_ACCS = 4;
+constexpr int FG_ACCS = 2;
+// The accumulators truncate, so every instruction that adds to them leaves a bias: 8e-9 of the result per k with three
+// instructions per slice in one accumulator (as on mma.sync), 5e-9 with the stacked form.  Up to this K the two stay
+// within 5e-6 of each other; beyond it the three-instruction form is kept, whose results are the mma.sync kernel's to 3e-6
+// (K = 12800) and which costs a fifth more operand reads.  Pointwise convolutions (short K, bound by HBM) keep it too: a
+// network binarises what follows them, and a sum that rounds the other way near zero flips a sign.
+constexpr int FG_STACKED_K = 2048;
 constexpr int FG_TILE_BYTES = 128 * 128;       // 128 rows x 32 floats
 constexpr int FG_STAGE_BYTES = 4 * FG_TILE_BYTES;   // pixels hi, pixels lo, weights hi, weights lo
 constexpr int FG_MAX_STAGES = 3;
@@ -36,8 +55,9 @@ __device__ __forceinline__ uint64_t fg_desc_sw128(uint32_t saddr) {
 
 __host__ __device__ inline int fg_smem_bytes(int stages) { return 1024 + stages * FG_STAGE_BYTES + 2 * FG_TILE_BYTES; }
 
+template <bool STACKED>
 __global__ void __launch_bounds__(FG_THREADS, 1)
-    fconv_gemm_kernel(const FconvParams p, const int M, const int stages, const int n_blk, const __grid_constant__ CUtensorMap a_map,
+    fconv_gemm_kernel(const FconvParams p, const int M, const int stages, const int n_blk, const int im2col, const __grid_constant__ CUtensorMap a_map,
                       const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap wr_map, const __grid_constant__ CUtensorMap out_map) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t bar_loaded[FG_MAX_STAGES], bar_ready[FG_MAX_STAGES], bar_empty[FG_MAX_STAGES];
@@ -49,12 +69,13 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
     unsigned char* stage0 = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
     unsigned char* stile = stage0 + stages * FG_STAGE_BYTES;
     const volatile int* abort_flag = &s_abort;
-    const int K = p.cin, nchunks = K / FG_CHUNK;
+    const int cgroups = (p.cin + FG_CHUNK - 1) / FG_CHUNK, taps = p.kh * p.kw, nchunks = taps * cgroups;
     // n_blk: channels per work item (32, 64 or 128: small when there are few pixel tiles, so that every SM gets work)
     const int tiles_m = (M + 127) / 128, nblocks = (p.cout + n_blk - 1) / n_blk;
     const uint32_t w_bytes = (uint32_t)n_blk * 128u;   // a weight tile of a stage
     const int nitems = tiles_m * nblocks;
-    constexpr int TMEM_COLS = FG_ACCS * FG_N;
+    constexpr int ACC_COLS = 2 * FG_N;                  // hi * W_hi + lo * W_hi in the first n_blk columns, hi * W_lo in the next
+    constexpr int TMEM_COLS = FG_ACCS * ACC_COLS;
 
     if (warp == FG_MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS));
@@ -82,6 +103,10 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
             bool ok = true;
             for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
                 const int tile = item / nblocks, nb = item - tile * nblocks;
+                // im2col: the window of the tile's first pixel starts here (input coordinates)
+                const int img = tile * 128 / (p.oh * p.ow), rem = tile * 128 - img * (p.oh * p.ow), oy = rem / p.ow, ox = rem - oy * p.ow;
+                const int y0 = oy * p.stride_h - p.pad_h, x0 = ox * p.stride_w - p.pad_w;
+                int cg = 0, tap = 0, ky = 0, kx = 0;
                 for (int c = 0; c < nchunks; c++) {
                     if (use >= 1 && !mbar_wait<32>(&bar_empty[s], (use - 1) & 1, abort_flag)) {
                         atomicCAS(&g_tc5_status, 0, 41);
@@ -91,14 +116,20 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                     }
                     const uint32_t bar = smem_u32(&bar_loaded[s]), sa = stage0_addr + s * FG_STAGE_BYTES;
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(FG_TILE_BYTES + (p.wgt_rem ? 2u : 1u) * w_bytes) : "memory");
-                    // rows beyond M / beyond Cout read as zeros; a load always delivers its whole box
-                    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                 ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&a_map)), "r"(c * FG_CHUNK), "r"(tile * 128), "r"(bar) : "memory");
-                    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                 ::"r"(sa + 2 * FG_TILE_BYTES), "l"(reinterpret_cast<uint64_t>(&w_map)), "r"(c * FG_CHUNK), "r"(nb * n_blk), "r"(bar) : "memory");
-                    if (p.wgt_rem)   // the weights' remainders were computed once, ahead of the launch
+                    // pixels beyond M, channels beyond Cin / Cout read as zeros; a load always delivers its whole box
+                    if (im2col)
+                        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6], {%7, %8};"
+                                     ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&a_map)), "r"(cg * FG_CHUNK), "r"(x0), "r"(y0), "r"(img), "r"(bar),
+                                       "h"((unsigned short)(kx * p.dil_w)), "h"((unsigned short)(ky * p.dil_h)) : "memory");
+                    else
                         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                     ::"r"(sa + 3 * FG_TILE_BYTES), "l"(reinterpret_cast<uint64_t>(&wr_map)), "r"(c * FG_CHUNK), "r"(nb * n_blk), "r"(bar) : "memory");
+                                     ::"r"(sa), "l"(reinterpret_cast<uint64_t>(&a_map)), "r"(cg * FG_CHUNK), "r"(tile * 128), "r"(bar) : "memory");
+                    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                                 ::"r"(sa + 2 * FG_TILE_BYTES), "l"(reinterpret_cast<uint64_t>(&w_map)), "r"(cg * FG_CHUNK), "r"(tap), "r"(nb * n_blk), "r"(bar) : "memory");
+                    if (p.wgt_rem)   // the weights' remainders were computed once, ahead of the launch
+                        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                                     ::"r"(sa + 2 * FG_TILE_BYTES + w_bytes), "l"(reinterpret_cast<uint64_t>(&wr_map)), "r"(cg * FG_CHUNK), "r"(tap), "r"(nb * n_blk), "r"(bar) : "memory");
+                    if (++cg == cgroups) { cg = 0; tap++; if (++kx == p.kw) { kx = 0; ky++; } }
                     if (++s == (uint32_t)stages) { s = 0; use++; }
                 }
             }
@@ -121,9 +152,9 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                 // 16-byte unit u of a hi tile -> the same unit of its lo tile (identical layouts)
 #pragma unroll
                 for (int half = 0; half < (p.wgt_rem ? 1 : 2); half++) {
-                    const uint32_t hi0 = sa + half * 2 * FG_TILE_BYTES + ct * 16, lo0 = hi0 + FG_TILE_BYTES;
-                    // eight units per thread and tile, their loads issued together (the shared-memory accesses are ordered
-                    // as written: one load, one store at a time would pay the load's latency eight times)
+                    const uint32_t hi0 = sa + half * 2 * FG_TILE_BYTES + ct * 16, lo0 = hi0 + (half ? w_bytes : (uint32_t)FG_TILE_BYTES);
+                    // four units per thread and tile, their loads issued together (the shared-memory accesses are ordered
+                    // as written: one load, one store at a time would pay the load's latency four times)
                     constexpr int UNITS = FG_TILE_BYTES / 16 / FG_CONVERTERS;
                     float4 v[UNITS];
 #pragma unroll
@@ -148,13 +179,12 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
             const uint32_t idesc_m = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(128 >> 4) << 24);   // D f32, A = B = tf32, K-major, M = 128
             const uint64_t d_stage = fg_desc_sw128(smem_u32(stage0));
             constexpr uint32_t TILE_UNITS = FG_TILE_BYTES >> 4, STAGE_UNITS = FG_STAGE_BYTES >> 4;
+            // weight rows beyond Cout read as zeros, so every item runs at the full width of its channel block
+            const uint32_t idesc = idesc_m | ((uint32_t)(n_blk >> 3) << 17), idesc2 = idesc_m | ((uint32_t)(n_blk >> 2) << 17);
             uint32_t s = 0, par = 0;
             bool ok = true;
             int i = 0;
             for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, i++) {
-                const int nb = item % nblocks;
-                const int n_mma = (min(n_blk, p.cout - nb * n_blk) + 15) & ~15;   // weight rows beyond Cout read as zeros
-                const uint32_t idesc = idesc_m | ((uint32_t)(n_mma >> 3) << 17);
                 const int accbuf = i % FG_ACCS, accuse = i / FG_ACCS;
                 if (accuse >= 1 && !mbar_wait(&bar_acc_empty[accbuf], (accuse - 1) & 1, abort_flag)) {
                     atomicCAS(&g_tc5_status, 0, 43);
@@ -162,8 +192,9 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d_tmem = tmem_base + accbuf * FG_N;
+                const uint32_t d_tmem = tmem_base + accbuf * ACC_COLS;
                 uint32_t accum = 0;
+                int cg = 0;
                 for (int c = 0; c < nchunks; c++) {
                     if (!mbar_wait(&bar_ready[s], par, abort_flag)) {
                         atomicCAS(&g_tc5_status, 0, 44);
@@ -172,13 +203,25 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ah = d_stage + (uint64_t)(s * STAGE_UNITS), al = ah + TILE_UNITS, wh = ah + 2 * TILE_UNITS, wl = ah + 3 * TILE_UNITS;
+                    const uint64_t ah = d_stage + (uint64_t)(s * STAGE_UNITS), al = ah + TILE_UNITS, wh = ah + 2 * TILE_UNITS, wl = wh + (w_bytes >> 4);
+                    auto slice = [&](int j) {   // 8 floats = 32 bytes along the swizzled row
+                        if (STACKED) {
+                            mma_tf32_ss(d_tmem, ah + 2 * j, wh + 2 * j, idesc2, j ? 1u : accum);
+                            mma_tf32_ss(d_tmem, al + 2 * j, wh + 2 * j, idesc, 1u);
+                        } else {
+                            mma_tf32_ss(d_tmem, ah + 2 * j, wh + 2 * j, idesc, j ? 1u : accum);
+                            mma_tf32_ss(d_tmem, ah + 2 * j, wl + 2 * j, idesc, 1u);
+                            mma_tf32_ss(d_tmem, al + 2 * j, wh + 2 * j, idesc, 1u);
+                        }
+                    };
+                    const int left = p.cin - cg * FG_CHUNK;
+                    if (left >= FG_CHUNK) {
 #pragma unroll
-                    for (int j = 0; j < FG_CHUNK / 8; j++) {   // 8 floats = 32 bytes along the swizzled row
-                        mma_tf32_ss(d_tmem, ah + 2 * j, wh + 2 * j, idesc, j ? 1u : accum);
-                        mma_tf32_ss(d_tmem, ah + 2 * j, wl + 2 * j, idesc, 1u);
-                        mma_tf32_ss(d_tmem, al + 2 * j, wh + 2 * j, idesc, 1u);
+                        for (int j = 0; j < FG_CHUNK / 8; j++) slice(j);
+                    } else {   // the last channel group of a tap: only the slices that hold channels
+                        for (int j = 0; j * 8 < left; j++) slice(j);
                     }
+                    if (++cg == cgroups) cg = 0;
                     accum = 1u;
                     umma_commit(&bar_empty[s]);
                     if (++s == (uint32_t)stages) { s = 0; par ^= 1u; }
@@ -211,11 +254,17 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                 uint32_t v[16];
                 if (okw && mine) {
                     const int c0 = cb + hq * 16;
-                    const uint32_t t_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + accbuf * FG_N + c0;
+                    const uint32_t t_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + accbuf * ACC_COLS + c0;
+                    uint32_t x[16] = {};
                     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
                                    "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                                  : "r"(t_addr));
+                    if (STACKED)
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]), "=r"(x[8]),
+                                   "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
+                                 : "r"(t_addr + n_blk));
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int q = 0; q < 4; q++) {   // channel constants four at a time (Cout is a multiple of four)
@@ -227,6 +276,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
 #pragma unroll
                         for (int e = 0; e < 4; e++) {
                             float f = __uint_as_float(v[q * 4 + e]);
+                            if (STACKED) f = __fadd_rn(f, __uint_as_float(x[q * 4 + e]));   // + the hi * W_lo part
                             if (p.bias) f = __fadd_rn(f, b4[e]);
                             if (p.a) f = __fadd_rn(__fmul_rn(a4[e], f), c4[e]);
                             if (p.relu) f = relu_ref(f);

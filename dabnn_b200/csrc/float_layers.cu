@@ -703,8 +703,23 @@ int fconv_split_weights(const float* weight, float* rem, size_t count, cudaStrea
     return check_launch("split_weights_kernel");
 }
 
+static bool fconv_is_pointwise(int kh, int kw, int pad_h, int pad_w, int stride_h, int stride_w) {
+    return kh == 1 && kw == 1 && stride_h == 1 && stride_w == 1 && pad_h == 0 && pad_w == 0;
+}
+
+// Shapes of the TMA-fed GEMM kernel: 16-byte channel rows, and windows within the im2col descriptor's fields (corner
+// offsets of a byte, tap offsets below 256, strides up to 8).  Thin inputs (below 16 channels would leave three quarters
+// of every 32-float row empty) stay with the kernels that stage input rows.
+static bool fconv_gemm_takes(int cin, int cout, int kh, int kw, int pad_h, int pad_w, int stride_h, int stride_w, int dil_h, int dil_w) {
+    if (cin % 4 || cout % 4 || cin < 16) return false;
+    if (fconv_is_pointwise(kh, kw, pad_h, pad_w, stride_h, stride_w)) return true;
+    const int far_h = pad_h - (kh - 1) * dil_h, far_w = pad_w - (kw - 1) * dil_w;
+    return stride_h <= 8 && stride_w <= 8 && pad_h <= 128 && pad_w <= 128 && far_h >= -128 && far_w >= -128 && far_h <= 127 && far_w <= 127 &&
+           (kh - 1) * dil_h < 256 && (kw - 1) * dil_w < 256;
+}
+
 bool fconv_uses_weight_remainders(int cin, int cout, int kh, int kw, int pad_h, int pad_w, int stride_h, int stride_w) {
-    return kh == 1 && kw == 1 && stride_h == 1 && stride_w == 1 && pad_h == 0 && pad_w == 0 && cin % FG_CHUNK == 0 && cout % 4 == 0;
+    return fconv_gemm_takes(cin, cout, kh, kw, pad_h, pad_w, stride_h, stride_w, 1, 1);
 }
 
 int fconv_impl(const float* in, const float* weight, const float* bias, const float* a, const float* b, int relu,
@@ -723,9 +738,10 @@ int fconv_impl(const float* in, const float* weight, const float* bias, const fl
     const FconvParams prm{in, weight, bias, a, b, out, relu, n, h, w, cin, cout, kh, kw, pad_h, pad_w,
                           stride_h, stride_w, dil_h, dil_w, oh, ow, (reinterpret_cast<uintptr_t>(weight_rem) & 15) == 0 ? weight_rem : nullptr};
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-    if (kh == 1 && kw == 1 && stride_h == 1 && stride_w == 1 && pad_h == 0 && pad_w == 0 && cin % FG_CHUNK == 0 && cout % 4 == 0 &&
-        al16(in) && al16(weight) && al16(out) && al16(bias) && al16(a) && al16(b)) {
-        // a 1x1 convolution is a GEMM over [pixels][cin]: TMA-fed (fconv_gemm.cuh)
+    const bool pointwise = fconv_is_pointwise(kh, kw, pad_h, pad_w, stride_h, stride_w);
+    if (fconv_gemm_takes(cin, cout, kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w) && al16(in) && al16(weight) && al16(out) && al16(bias) &&
+        al16(a) && al16(b)) {
+        // a GEMM over (taps, channels), fed by TMA (fconv_gemm.cuh)
         static thread_local int gemm_device = -1, gemm_stages = 0;
         int dev = 0;
         DABNN_CUDA_OK(cudaGetDevice(&dev));
@@ -733,28 +749,36 @@ int fconv_impl(const float* in, const float* weight, const float* bias, const fl
             int optin = 0;
             cudaFuncAttributes fa;
             DABNN_CUDA_OK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-            DABNN_CUDA_OK(cudaFuncGetAttributes(&fa, fconv_gemm_kernel));
+            DABNN_CUDA_OK(cudaFuncGetAttributes(&fa, fconv_gemm_kernel<true>));
             gemm_stages = FG_MAX_STAGES;
             while (gemm_stages >= 2 && fg_smem_bytes(gemm_stages) > optin - (int)fa.sharedSizeBytes) gemm_stages--;
-            if (gemm_stages >= 2)
-                DABNN_CUDA_OK(cudaFuncSetAttribute(fconv_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fg_smem_bytes(gemm_stages)));
+            if (gemm_stages >= 2) {
+                DABNN_CUDA_OK(cudaFuncSetAttribute(fconv_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, fg_smem_bytes(gemm_stages)));
+                DABNN_CUDA_OK(cudaFuncSetAttribute(fconv_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fg_smem_bytes(gemm_stages)));
+            }
             gemm_device = dev;
         }
         const int Mpx = n * oh * ow, tiles_m = (Mpx + 127) / 128;
-        // channels per work item: as large as leaves every SM a work item
-        int n_blk = FG_N;
-        while (n_blk > 32 && tiles_m * ((cout + n_blk - 1) / n_blk) < sm_count()) n_blk >>= 1;
+        // channels per work item: equal blocks of at most 128 (in 32s, the width of a store's box), smaller ones where they
+        // would leave SMs without a work item
+        const int blocks = (cout + FG_N - 1) / FG_N;
+        int n_blk = ((cout + blocks - 1) / blocks + 31) & ~31;
+        while (n_blk > 32 && tiles_m * ((cout + n_blk - 1) / n_blk) < sm_count()) n_blk = (n_blk / 2 + 31) & ~31;
         CUtensorMap a_map, w_map, wr_map{}, o_map;
-        const unsigned box[2] = {32, 128}, wbox[2] = {32, (unsigned)n_blk};
-        const unsigned long long adims[2] = {(unsigned long long)cin, (unsigned long long)Mpx}, astr[1] = {(unsigned long long)cin * 4};
-        const unsigned long long wdims[2] = {(unsigned long long)cin, (unsigned long long)cout};
+        const unsigned long long row = (unsigned long long)cin * 4;
+        const unsigned box[2] = {FG_CHUNK, 128}, wbox[3] = {FG_CHUNK, 1, (unsigned)n_blk};
+        const unsigned long long adims[2] = {(unsigned long long)cin, (unsigned long long)Mpx}, astr[1] = {row};
+        const unsigned long long wdims[3] = {(unsigned long long)cin, (unsigned long long)kh * kw, (unsigned long long)cout}, wstr[2] = {row, row * kh * kw};
         const unsigned long long odims[2] = {(unsigned long long)cout, (unsigned long long)Mpx}, ostr[1] = {(unsigned long long)cout * 4};
-        if (gemm_stages >= 2 && make_f32_tensor_map(&a_map, const_cast<float*>(in), 2, adims, astr, box) &&
-            make_f32_tensor_map(&w_map, const_cast<float*>(weight), 2, wdims, astr, wbox) && make_f32_tensor_map(&o_map, out, 2, odims, ostr, box) &&
-            (!prm.wgt_rem || make_f32_tensor_map(&wr_map, const_cast<float*>(prm.wgt_rem), 2, wdims, astr, wbox))) {
+        const bool have_a = pointwise ? make_f32_tensor_map(&a_map, const_cast<float*>(in), 2, adims, astr, box)
+                                      : make_f32_im2col_map(&a_map, in, n, h, w, cin, kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, FG_CHUNK, 128);
+        if (gemm_stages >= 2 && have_a && make_f32_tensor_map(&w_map, const_cast<float*>(weight), 3, wdims, wstr, wbox) &&
+            make_f32_tensor_map(&o_map, out, 2, odims, ostr, box) &&
+            (!prm.wgt_rem || make_f32_tensor_map(&wr_map, const_cast<float*>(prm.wgt_rem), 3, wdims, wstr, wbox))) {
             const int items = tiles_m * ((cout + n_blk - 1) / n_blk);
-            launch_overlapped(fconv_gemm_kernel, std::min(items, sm_count()), FG_THREADS, fg_smem_bytes(gemm_stages), stream, prm, Mpx, gemm_stages, n_blk, a_map,
-                              w_map, wr_map, o_map);
+            const bool stacked = !pointwise && kh * kw * ((cin + FG_CHUNK - 1) / FG_CHUNK) * FG_CHUNK <= FG_STACKED_K;
+            launch_overlapped(stacked ? fconv_gemm_kernel<true> : fconv_gemm_kernel<false>, std::min(items, sm_count()), FG_THREADS,
+                              fg_smem_bytes(gemm_stages), stream, prm, Mpx, gemm_stages, n_blk, (int)!pointwise, a_map, w_map, wr_map, o_map);
             return check_launch("fconv_gemm_kernel");
         }
     }

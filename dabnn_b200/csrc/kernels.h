@@ -16,6 +16,11 @@ namespace dabnn {
 bool make_f32_tensor_map(CUtensorMap_st* map, float* base, int rank, const unsigned long long* dims,
                          const unsigned long long* strides_bytes, const unsigned* box);
 
+// The same for im2col-mode loads of an fp32 NHWC tensor: `pixels` consecutive output positions of a convolution window
+// (n outermost), `channels` floats each, 128-byte-swizzled.
+bool make_f32_im2col_map(CUtensorMap_st* map, const float* base, int n, int h, int w, int c, int kh, int kw, int pad_h, int pad_w, int stride_h,
+                         int stride_w, int dil_h, int dil_w, int channels, int pixels);
+
 // The same for a tensor of bytes, up to five dimensions, inner box 64 or 128 bytes, swizzled over that width (the
 // layout a K-major SWIZZLE_64B / SWIZZLE_128B shared-memory descriptor of tcgen05.mma reads); elements outside the
 // tensor read as zero.

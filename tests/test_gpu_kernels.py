@@ -469,6 +469,31 @@ def test_fconv_dilation(ops, port, h, cin, cout, ks, stride, pad, dil):
     assert ops.engine_status() == 0
 
 
+@pytest.mark.parametrize("n,h,w,cin,cout,ks,stride,pad,dil,bias", [
+    (1, 8, 16, 32, 32, 3, 1, 1, 1, True),      # exactly one 128-pixel tile
+    (1, 43, 3, 32, 16, 3, 1, 1, 1, False),     # 129 pixels: a tile of one
+    (3, 9, 7, 20, 36, 3, 2, 1, 1, True),       # a partial channel group, channels that end inside a store's box, stride 2
+    (2, 11, 6, 48, 144, 5, 1, 2, 1, True),     # two channel groups (the second half empty), two channel blocks
+    (2, 15, 13, 16, 20, 3, 1, 2, 2, False),    # dilation
+    (3, 6, 5, 36, 8, 1, 2, 0, 1, True),        # pointwise with stride
+    (2, 4, 4, 64, 40, 4, 1, 0, 1, True),       # the window is the image (a fully connected layer)
+    (40, 24, 24, 16, 128, 3, 1, 1, 1, True),   # more tiles than SMs: every CTA's ring and accumulators wrap
+    (2, 9, 9, 232, 64, 3, 1, 1, 1, True),      # K above the stacked form's limit
+])
+def test_fconv_im2col_gemm(ops, port, n, h, w, cin, cout, ks, stride, pad, dil, bias):
+    """Windows on the TMA-fed GEMM kernel (dabnn/fconv.h:14-76).  The accumulators truncate: at most 1e-8 of the summed
+    magnitudes per k, 2.1e-5 at the largest K here, below the 1e-4 every float layer is held to."""
+    rng = np.random.default_rng(h * cin + ks)
+    x = rng.normal(0, 1, (n, h, w, cin)).astype(np.float32)
+    wt = rng.normal(0, np.sqrt(2.0 / (cin * ks * ks)), (cout, ks, ks, cin)).astype(np.float32)
+    bv = rng.normal(0, 1, cout).astype(np.float32) if bias else None
+    out = host(ops.fconv(dev_f32(x), dev_f32(wt), dev_f32(bv) if bias else None, pad, pad, stride, stride, dil, dil))
+    for i in {0, n // 2, n - 1}:
+        exp = port.fconv(x[i], wt, bv, pad, pad, stride, stride, dil, dil)
+        np.testing.assert_allclose(out[i], exp, rtol=1e-4, atol=1e-4 * float(np.abs(exp).max()))
+    assert ops.engine_status() == 0
+
+
 @pytest.mark.parametrize("cin,cout,ks", [(64, 64, 3), (128, 32, 3), (64, 128, 1), (256, 64, 3)])
 def test_batchnorm_fold_identity(ops, port, cin, cout, ks):
     """The converter's BatchNorm fold for a binary convolution (reference tools/onnx2bnn/OnnxConverter.cpp:583-639:
