@@ -81,6 +81,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
     }
     return false;
 }
+// the same for a whole warp: every lane gets the same answer
+template <int SLEEP_NS = 0>
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait<SLEEP_NS>(bar, parity, abort_flag));
+}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }

@@ -23,11 +23,11 @@
 // into one slot; 98 of the MMA's 128 rows carry pixels, and the nine taps of a pixel cost one load instead of nine.
 //
 // A block whose result also feeds a 2x2 stride-2 average pooling (the downsample shortcut of the next stage: reference
-// layers/AvePool.cpp:84) can write the pooled tensor as well: tiles are then an even number of output rows, and after a
-// block of 64 channels is staged every thread folds one pooled pixel x four channels out of the staging tile, in the
-// reference's tap order, sum first, then the division.
+// layers/AvePool.cpp:84) can write the pooled tensor as well: tiles are then an even number of output rows, the
+// four warps of an item leave their results in their buffers and, between two barriers of their own, fold pooled pixels x
+// four channels out of them in the reference's tap order, sum first, then the division.
 //
-// Warps: 0 halo loads, 1 weight loads, 2 MMA issue (one lane each), 3 .. 18 epilogue (as in bconv_u8.cuh, with the
+// Warps: 0 halo loads, 1 weight loads, 2 MMA issue (one lane each), 3 .. 14 epilogue (bconv_epilogue.cuh, with the
 // accumulator row -> pixel mapping above).  Every wait is bounded; a wait that gives up records a code in the
 // byte-activation engine's status word (21 halo loader, 25 weight loader, 22 / 23 / 26 MMA thread waiting for an
 // accumulator / a halo / a weight stage, 24 epilogue), raises the CTA's abort flag, and the CTA frees its tensor
@@ -37,7 +37,7 @@
 
 namespace dabnn {
 
-constexpr int HL_THREADS = 96 + U8_EPILOGUE;   // warps 0, 1, 2 + the epilogue warps
+constexpr int HL_THREADS = 96 + EPI_THREADS;   // warps 0, 1, 2 + the epilogue warps
 constexpr int HL_MAX_HSLOTS = 8, HL_MAX_WSTAGES = 8;   // (more than four weight stages only with narrow channel blocks)
 
 struct HaloParams {
@@ -58,25 +58,23 @@ struct HaloParams {
     int wb;                       // rows of a weight box image
     int nb;                       // output channels per CTA: TC5_MAX_N, or 64 / 32 when there are too few tiles to fill the SMs
                                   // (streamed weights only: a CTA then copies its rows out of every box image)
-    int resident, stiles, pair;
-    int lag;                      // tensor stores that may still be reading their staging tile when the next shortcut is fetched (0 or 1):
-                                  // the shortcut runs stiles - 1 - lag blocks ahead
+    int resident, pair;
+    int narrow;                   // see EpiOut
 };
 
-template <bool PAIR>
+template <bool PAIR, bool POOL>
 __global__ void __launch_bounds__(HL_THREADS, 1)
-    bconv_halo_kernel(const HaloParams p, const __grid_constant__ CUtensorMap in_map, const __grid_constant__ CUtensorMap out_map,
-                      const __grid_constant__ CUtensorMap sc_map) {
+    bconv_halo_kernel(const HaloParams p, const __grid_constant__ CUtensorMap in_map) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t halo_full[HL_MAX_HSLOTS], halo_empty[HL_MAX_HSLOTS], w_full[HL_MAX_WSTAGES], w_empty[HL_MAX_WSTAGES];
-    __shared__ __align__(8) uint64_t bar_acc_full[U8_ACCS], bar_acc_empty[U8_ACCS], bar_w, sc_full[U8_MAX_STILES];
+    __shared__ __align__(8) uint64_t bar_acc_full[U8_ACCS], bar_acc_empty[U8_ACCS], bar_w;
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_abort, epi_abort;
-    __shared__ __align__(16) int popw[TC5_MAX_N];
+    __shared__ __align__(16) float pop[TC5_MAX_N];
     __shared__ __align__(16) float chan_a[TC5_MAX_N];
     __shared__ __align__(16) float chan_b[TC5_MAX_N];
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int n0 = blockIdx.y * p.nb;
     const int n_this = min(p.nb, p.N - n0);        // multiple of 16 (host-checked)
     const int n_mma = n_this;
@@ -85,12 +83,11 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
     const int nboxes = 9 * p.cw, gbox_bytes = p.wb * 64, wbox_bytes = min(p.nb, p.wb) * 64;   // a box image in global / this CTA's rows of it
     unsigned char* halo0 = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
     unsigned char* wbase = halo0 + p.hslots * p.halo_stride;                                   // resident weights or the weight ring
-    unsigned char* sbuf0 = wbase + (p.resident ? nboxes * wbox_bytes : p.wstages * 3 * wbox_bytes);   // a multiple of 1024 bytes further
+    unsigned char* epi_buf = wbase + (p.resident ? nboxes * wbox_bytes : p.wstages * 3 * wbox_bytes);   // a multiple of 1024 bytes further
+    const int acc_cols = (n_mma + 31) & ~31;       // columns between accumulators: whole 32-column items
     int tmem_cols = 32;
-    while (tmem_cols < U8_ACCS * n_mma) tmem_cols <<= 1;
+    while (tmem_cols < U8_ACCS * acc_cols) tmem_cols <<= 1;
     const volatile int* abort_flag = &s_abort;
-    const int box_px = p.imgs * p.rows * p.OW;      // pixels a tile's stores cover
-    const int srows = u8_staging_rows(box_px), sbox_bytes = srows * 128, stile_bytes = 2 * sbox_bytes;
     const uint32_t halo_tx = (uint32_t)(p.imgs * (p.rows + 2) * p.P * 64);
 
     if (warp == 2) {
@@ -100,9 +97,8 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
     if (tid == 0) {
         for (int i = 0; i < p.hslots; i++) { mbar_init(&halo_full[i], 1); mbar_init(&halo_empty[i], 1); }
         for (int i = 0; i < HL_MAX_WSTAGES; i++) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], 1); }
-        for (int i = 0; i < U8_ACCS; i++) { mbar_init(&bar_acc_full[i], 1); mbar_init(&bar_acc_empty[i], U8_EPI_WARPS); }
+        for (int i = 0; i < U8_ACCS; i++) { mbar_init(&bar_acc_full[i], 1); mbar_init(&bar_acc_empty[i], 4 * ((n_this + 31) >> 5)); }
         mbar_init(&bar_w, 1);
-        for (int i = 0; i < U8_MAX_STILES; i++) mbar_init(&sc_full[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::);
         s_abort = 0;
         epi_abort = 0;
@@ -110,7 +106,7 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
     if (p.imgs == 2 && tid < p.hslots * 4)   // the zero pixel behind the second image's halo (never written again)
         sts128(smem_u32(halo0) + (tid >> 2) * p.halo_stride + (p.img_pitch + (p.rows + 2) * p.P) * 64 + (tid & 3) * 16, 0u, 0u, 0u, 0u);
     if (tid < TC5_MAX_N) {
-        popw[tid] = tid < n_this ? __ldg(reinterpret_cast<const int*>(p.w_img + u8_weight_image_bytes(p.N, nboxes)) + n0 + tid) : 0;
+        pop[tid] = (tid < n_this ? (float)__ldg(reinterpret_cast<const int*>(p.w_img + u8_weight_image_bytes(p.N, nboxes)) + n0 + tid) : 0.f) - EPI_POP_BIAS;
         const bool have = p.a && tid < n_this;
         chan_a[tid] = have ? __ldg(p.a + n0 + tid) : 1.f;
         chan_b[tid] = have ? __ldg(p.b + n0 + tid) : 0.f;
@@ -188,63 +184,64 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
             }
         }
     } else if (warp == 2) {
-        // =========================== MMA issue: one lane ===========================
-        if (lane == 0) {
-            // instruction descriptor: D = s32, A = u8, B = s8, both K-major, N = n_mma, M = 128
-            const uint32_t idesc = (2u << 4) | (1u << 10) | ((uint32_t)(n_mma >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-            const uint64_t d_halo = umma_desc_sw64(smem_u32(halo0));
-            const uint64_t d_w = umma_desc(smem_u32(wbase), 512);
-            const uint32_t halo_units = (uint32_t)p.halo_stride >> 4, wbox_units = (uint32_t)wbox_bytes >> 4, row_units = (uint32_t)p.P * 4u;
-            bool ok = true;
-            if (p.resident && !mbar_wait(&bar_w, 0, abort_flag)) {
-                atomicCAS(&g_u8_status, 0, 26);
-                s_abort = 1;
-                ok = false;
+        // =========================== MMA issue: the whole warp walks, one lane issues ===========================
+        // instruction descriptor: D = s32, A = u8, B = s8, both K-major, N = n_mma, M = 128
+        const uint32_t idesc = (2u << 4) | (1u << 10) | ((uint32_t)(n_mma >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint64_t d_halo = umma_desc_sw64(smem_u32(halo0));
+        const uint64_t d_w = umma_desc(smem_u32(wbase), 512);
+        const uint32_t halo_units = (uint32_t)p.halo_stride >> 4, wbox_units = (uint32_t)wbox_bytes >> 4, row_units = (uint32_t)p.P * 4u;
+        const bool leader = elect_lane();
+        bool ok = true;
+        if (p.resident && !mbar_wait_warp(&bar_w, 0, abort_flag)) {
+            atomicCAS(&g_u8_status, 0, 26);
+            s_abort = 1;
+            ok = false;
+        }
+        uint32_t hs = 0, hpar = 0, ws = 0, wpar = 0;
+        int i = 0;   // tiles so far: tile i accumulates in accumulator i % U8_ACCS
+        for (int unit = blockIdx.x; unit < nunits && ok; unit += gridDim.x, i += np) {
+            for (int t = 0; t < np && ok; t++) {
+                const int accbuf = (i + t) % U8_ACCS, accuse = (i + t) / U8_ACCS;
+                if (accuse >= 1 && !mbar_wait_warp(&bar_acc_empty[accbuf], (accuse - 1) & 1, abort_flag)) {
+                    atomicCAS(&g_u8_status, 0, 22);
+                    s_abort = 1;
+                    ok = false;
+                }
             }
-            uint32_t hs = 0, hpar = 0, ws = 0, wpar = 0;
-            int i = 0;   // tiles so far: tile i accumulates in accumulator i % U8_ACCS
-            for (int unit = blockIdx.x; unit < nunits && ok; unit += gridDim.x, i += np) {
-                for (int t = 0; t < np && ok; t++) {
-                    const int accbuf = (i + t) % U8_ACCS, accuse = (i + t) / U8_ACCS;
-                    if (accuse >= 1 && !mbar_wait(&bar_acc_empty[accbuf], (accuse - 1) & 1, abort_flag)) {
-                        atomicCAS(&g_u8_status, 0, 22);
+            if (!ok) break;
+            uint32_t d_tmem[np];
+            for (int t = 0; t < np; t++) d_tmem[t] = tmem_base + ((i + t) % U8_ACCS) * acc_cols;
+            uint32_t accum = 0;
+            for (int cg = 0; cg < p.cw && ok; cg++) {
+                uint32_t slot[np];
+                for (int t = 0; t < np; t++) {   // this group's halo of every tile of the unit
+                    if (!mbar_wait_warp(&halo_full[hs], hpar, abort_flag)) {
+                        atomicCAS(&g_u8_status, 0, 23);
                         s_abort = 1;
                         ok = false;
+                        break;
                     }
+                    slot[t] = hs;
+                    if (++hs == (uint32_t)p.hslots) { hs = 0; hpar ^= 1u; }
                 }
                 if (!ok) break;
-                uint32_t d_tmem[np];
-                for (int t = 0; t < np; t++) d_tmem[t] = tmem_base + ((i + t) % U8_ACCS) * n_mma;
-                uint32_t accum = 0;
-                for (int cg = 0; cg < p.cw && ok; cg++) {
-                    uint32_t slot[np];
-                    for (int t = 0; t < np; t++) {   // this group's halo of every tile of the unit
-                        if (!mbar_wait(&halo_full[hs], hpar, abort_flag)) {
-                            atomicCAS(&g_u8_status, 0, 23);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int ky = 0; ky < 3; ky++) {
+                    uint64_t bd;
+                    if (p.resident) {
+                        bd = d_w + (uint64_t)((ky * 3 * p.cw + cg) * wbox_units);
+                    } else {
+                        if (!mbar_wait_warp(&w_full[ws], wpar, abort_flag)) {
+                            atomicCAS(&g_u8_status, 0, 26);
                             s_abort = 1;
                             ok = false;
                             break;
                         }
-                        slot[t] = hs;
-                        if (++hs == (uint32_t)p.hslots) { hs = 0; hpar ^= 1u; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        bd = d_w + (uint64_t)(ws * 3 * wbox_units);
                     }
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (int ky = 0; ky < 3; ky++) {
-                        uint64_t bd;
-                        if (p.resident) {
-                            bd = d_w + (uint64_t)((ky * 3 * p.cw + cg) * wbox_units);
-                        } else {
-                            if (!mbar_wait(&w_full[ws], wpar, abort_flag)) {
-                                atomicCAS(&g_u8_status, 0, 26);
-                                s_abort = 1;
-                                ok = false;
-                                break;
-                            }
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            bd = d_w + (uint64_t)(ws * 3 * wbox_units);
-                        }
-                        const uint32_t bstep = p.resident ? (uint32_t)p.cw * wbox_units : wbox_units;   // from tap kx to tap kx + 1
+                    const uint32_t bstep = p.resident ? (uint32_t)p.cw * wbox_units : wbox_units;   // from tap kx to tap kx + 1
+                    if (leader) {
 #pragma unroll
                         for (int t = 0; t < np; t++) {
                             // tap (ky, kx): the halo read from pixel ky * P + kx on; 32 bytes of K per MMA
@@ -255,197 +252,128 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
                                 mma_i8_ss(d_tmem[t], ad + kx * 4 + 2, bd + kx * bstep + 16, idesc, 1u);
                             }
                         }
-                        accum = 1u;
-                        if (!p.resident) {
-                            umma_commit(&w_empty[ws]);
-                            if (++ws == (uint32_t)p.wstages) { ws = 0; wpar ^= 1u; }
-                        }
+                        if (!p.resident) umma_commit(&w_empty[ws]);
                     }
-                    if (ok)
-                        for (int t = 0; t < np; t++) umma_commit(&halo_empty[slot[t]]);
+                    accum = 1u;
+                    if (!p.resident && ++ws == (uint32_t)p.wstages) { ws = 0; wpar ^= 1u; }
                 }
-                if (ok)
-                    for (int t = 0; t < np; t++) umma_commit(&bar_acc_full[(i + t) % U8_ACCS]);
+                if (ok && leader)
+                    for (int t = 0; t < np; t++) umma_commit(&halo_empty[slot[t]]);
             }
+            if (ok && leader)
+                for (int t = 0; t < np; t++) umma_commit(&bar_acc_full[(i + t) % U8_ACCS]);
+            __syncwarp();
         }
     } else {
         // =========================== epilogue ===========================
-        // As in bconv_u8.cuh: blocks of 64 channels through p.stiles fp32 staging tiles, the shortcut prefetched by cp.async,
-        // one TMA tensor store per 32-channel box, sign bytes and packed bits straight from registers.  Accumulator row r is
-        // halo pixel r: output row r / P of the tile, column r % P; it has a pixel when the column is below OW.
-        const int et = tid - 96, ew = warp - 3;
-        const int r = (warp & 3) * 32 + lane, hq = ew >> 2;   // TMEM lane quarter of a warp = warp % 4; column quarter 0..3
-        const int second = (p.imgs == 2 && r >= p.img_pitch) ? 1 : 0, rr = r - second * p.img_pitch;   // which image of the tile
-        const int orow = rr / p.P, ocol = rr - orow * p.P;
-        const bool has_px = ocol < p.OW && orow < p.rows;
-        const int m = (second * p.rows + orow) * p.OW + ocol;   // the pixel's index within the tile (dense), its staging row
-        const uint32_t sbuf0_addr = smem_u32(sbuf0);
-        const int nblk = (n_this + 63) >> 6;
-        const int first_tile = blockIdx.x * np;
-        auto next_tile = [&](int tile, int index) {   // the tile after `tile`, which is this CTA's tile number `index`
-            return np == 1 ? tile + (int)gridDim.x : ((index & 1) ? tile + 2 * (int)gridDim.x - 1 : tile + 1);
-        };
-        int my_tiles = 0;
-        for (int t = first_tile, k = 0; t < p.ntiles; t = next_tile(t, k++)) my_tiles++;
-        const int total_blocks = my_tiles * nblk;
-        auto tile_span = [&](int tile, long long& base, int& nvalid, int& img0, int& oh0) {
+        // Accumulator row r is halo pixel r: output row r / P of the tile, column r % P; it has a pixel when the column is
+        // below OW.
+        const int ew = warp - 3, group = ew >> 2, r0 = (warp & 3) * 32;   // TMEM lane quarter of a warp = warp % 4
+        EpiWarp e;
+        const uint32_t epi_addr = smem_u32(epi_buf);
+        e.init(epi_addr, ew);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int r = r0 + e.row_of(k);
+            const int second = (p.imgs == 2 && r >= p.img_pitch) ? 1 : 0, rr = r - second * p.img_pitch;   // which image of the tile
+            const int orow = rr / p.P, ocol = rr - orow * p.P;
+            e.set_row(k, ocol < p.OW && orow < p.rows ? (second * p.rows + orow) * p.OW + ocol : -1, p.N);   // the pixel's index within the tile
+        }
+        const EpiOut o{p.out, p.out_u8, p.out_bits, p.narrow};
+        const EpiChannels ch{pop, chan_a, chan_b};
+        // Items: 32-channel chunks of this CTA's tiles in order, dealt to the warp groups in turn.
+        const int nchunk = (n_this + 31) >> 5;
+        const EpiDiv per_img(p.tiles_per_img, p.ntiles + (int)gridDim.x * 16);
+        auto tile_of = [&](int k) { return (blockIdx.x + (k / np) * (int)gridDim.x) * np + k % np; };      // this CTA's k-th tile
+        auto tile_span = [&](int tile, long long& base, int& nvalid) {
             if (p.imgs == 2) {   // whole images, the last tile may hold one
-                img0 = tile * 2; oh0 = 0;
-                base = (long long)img0 * p.OH * p.OW;
-                nvalid = max(0, min(2, p.B - img0)) * p.OH * p.OW;
+                base = (long long)tile * 2 * p.OH * p.OW;
+                nvalid = max(0, min(2, p.B - tile * 2)) * p.OH * p.OW;
                 return;
             }
-            img0 = tile / p.tiles_per_img; oh0 = (tile - img0 * p.tiles_per_img) * p.rows;
-            base = ((long long)img0 * p.OH + oh0) * p.OW;
+            const int img = per_img(tile), oh0 = (tile - img * p.tiles_per_img) * p.rows;
+            base = ((long long)img * p.OH + oh0) * p.OW;
             nvalid = min(p.rows, p.OH - oh0) * p.OW;
         };
-        // The shortcut of block kb + stiles - 1 is fetched into the staging tile that block kb - 1 has left, by one thread and
-        // two tiled TMA loads (the tile's layout is the one the tensor store reads, so the sum happens in place).
-        int pkb = 0, ptile = first_tile, pti = 0, pblk = 0, pst = 0;
-        auto prefetch_next = [&]() {   // thread et == 0 only
-            if (p.shortcut && pkb < total_blocks) {
-                const int pimg = p.imgs == 2 ? ptile * 2 : ptile / p.tiles_per_img, poh0 = p.imgs == 2 ? 0 : (ptile - pimg * p.tiles_per_img) * p.rows;
-                const int cb = pblk * 64, boxes = n_this - cb > 32 ? 2 : 1;
-                const uint32_t bar = smem_u32(&sc_full[pst]), dst = sbuf0_addr + pst * stile_bytes;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)(boxes * box_px * 128)) : "memory");
-                for (int hb = 0; hb < boxes; hb++)
-                    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                                 ::"r"(dst + hb * sbox_bytes), "l"(reinterpret_cast<uint64_t>(&sc_map)), "r"(n0 + cb + hb * 32), "r"(poh0 * p.OW), "r"(pimg),
-                                   "r"(bar) : "memory");
-            }
-            pkb++;
-            if (++pst == p.stiles) pst = 0;
-            if (++pblk == nblk) {
-                pblk = 0;
-                ptile = next_tile(ptile, pti++);
-            }
-        };
-        if (et == 0)
-            for (int d = 0; d + 1 + p.lag < p.stiles; d++) prefetch_next();
-        bool okw = true;
-        uint32_t sc_par = 0;
-        int tile = first_tile, ti = 0, blk = 0, st_idx = 0, accbuf = 0, accuse = 0, nvalid = 0, img0 = 0, oh0 = 0;
+        auto element = [&](long long base, int chunk) { return (size_t)base * p.N + n0 + chunk * 32 + e.q * 8; };   // of a tile's first pixel, at the lane's channels
+        auto limit_of = [&](int nvalid, int chunk) { return chunk * 32 + e.q * 8 < n_this ? (uint32_t)(nvalid * p.N) : 0u; };
+        int k = group / nchunk, chunk = group - k * nchunk, tile = tile_of(k);
         long long base = 0;
-        for (int kb = 0; kb < total_blocks; kb++) {
-            if (blk == 0) tile_span(tile, base, nvalid, img0, oh0);
-            const int cb = blk * 64;
-            const int width = min(64, n_this - cb);
-            const uint32_t sb = sbuf0_addr + st_idx * stile_bytes;
-            if (et == 0) {   // the tile the next shortcut goes to is idle once the stores of block kb - 1 - lag have read it
-                if (p.lag) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                prefetch_next();
-            }
-            if (p.shortcut && okw) {   // the shortcut of block kb has landed in its tile
-                okw = __all_sync(0xffffffffu, mbar_wait<100>(&sc_full[st_idx], sc_par, abort_flag));
-                if (!okw) {
-                    atomicCAS(&g_u8_status, 0, 24);
-                    s_abort = 1;
-                    epi_abort = 1;
-                }
-            }
-            const bool mine = width > hq * 16;                               // this thread's 16 columns exist
-            if (blk == 0 && okw) {
-                okw = __all_sync(0xffffffffu, mbar_wait<200>(&bar_acc_full[accbuf], accuse & 1, abort_flag));
-                if (!okw) {
-                    atomicCAS(&g_u8_status, 0, 24);
-                    s_abort = 1;
-                    epi_abort = 1;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            }
-            if (okw && mine) {
-                const int c0 = cb + hq * 16;
-                const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + accbuf * n_mma;
-                uint32_t v[16];
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                               "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                             : "r"(t_row + c0));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const bool valid = has_px && m < nvalid;   // the last tile of an image may have fewer rows
-                if (valid) {
-                    // chunk qq (4 channels) of this pixel's row in box hq / 2: srow + ((qq ^ (m & 7)) << 4)
-                    const uint32_t srow = sb + (hq >> 1) * sbox_bytes + m * 128;
-                    uint32_t signs = 0;   // bit j: channel c0 + j of this pixel is positive
+        int nvalid = 0;
+        if (tile < p.ntiles) {
+            tile_span(tile, base, nvalid);
+            if (p.shortcut) {
+                const float* at = p.shortcut + element(base, chunk);
+                const uint32_t limit = limit_of(nvalid, chunk);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int cl = c0 + q * 4;
-                        const int4 pw = *reinterpret_cast<const int4*>(popw + cl);
-                        float o[4];
-                        o[0] = small_int_to_float(pw.x + (int)v[q * 4 + 0]);
-                        o[1] = small_int_to_float(pw.y + (int)v[q * 4 + 1]);
-                        o[2] = small_int_to_float(pw.z + (int)v[q * 4 + 2]);
-                        o[3] = small_int_to_float(pw.w + (int)v[q * 4 + 3]);
-                        if (p.a) {
-                            const float4 ca = *reinterpret_cast<const float4*>(chan_a + cl), cbv = *reinterpret_cast<const float4*>(chan_b + cl);
-                            o[0] = __fadd_rn(__fmul_rn(ca.x, o[0]), cbv.x); o[1] = __fadd_rn(__fmul_rn(ca.y, o[1]), cbv.y);
-                            o[2] = __fadd_rn(__fmul_rn(ca.z, o[2]), cbv.z); o[3] = __fadd_rn(__fmul_rn(ca.w, o[3]), cbv.w);
-                        }
-                        const uint32_t sa = srow + ((((hq & 1) * 4 + q) ^ (m & 7)) << 4);
-                        if (p.shortcut) {
-                            const float4 ad = lds128f(sa);
-                            o[0] = __fadd_rn(ad.x, o[0]); o[1] = __fadd_rn(ad.y, o[1]);
-                            o[2] = __fadd_rn(ad.z, o[2]); o[3] = __fadd_rn(ad.w, o[3]);
-                        }
-                        sts128f(sa, o[0], o[1], o[2], o[3]);
-                        signs |= ((o[0] > 0.f ? 1u : 0u) | (o[1] > 0.f ? 2u : 0u) | (o[2] > 0.f ? 4u : 0u) | (o[3] > 0.f ? 8u : 0u)) << (q * 4);
-                    }
-                    const long long row = base + m;
-                    if (p.out_bits)   // 16 channels = a quarter of a packed word (a narrow channel block may start inside a word)
-                        reinterpret_cast<unsigned short*>(p.out_bits + row * (p.N >> 6) + ((n0 + cb) >> 6))[(((n0 + cb) & 63) >> 4) + hq] = (unsigned short)signs;
-                    if (p.out_u8) {
-                        uint32_t w8[4];
-#pragma unroll
-                        for (int q = 0; q < 4; q++) w8[q] = (((signs >> (q * 4)) & 0xfu) * 0x00204081u) & 0x01010101u;
-                        *reinterpret_cast<uint4*>(p.out_u8 + row * p.N + n0 + c0) = make_uint4(w8[0], w8[1], w8[2], w8[3]);
-                    }
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor store below reads what was just written
-            }
-            if (blk == nblk - 1 && okw) {   // the whole accumulator has been read
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_acc_empty[accbuf]);
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(U8_EPILOGUE) : "memory");   // results of block kb are staged (or abort decided)
-            if (epi_abort) break;
-            // ---- write-out: one tensor store per 32-channel box; pixels beyond the image and channels beyond N are clipped ----
-            if (p.pool_out) {
-                // 2x2 average pooling of the staged block: task = pooled pixel (prow, pcol) x four channels
-                const int pw = p.OW >> 1, q = et & 15, pp = et >> 4;
-                const int prow = pp / pw, pcol = pp - prow * pw;
-                if (prow < (p.rows >> 1) && (2 * prow + 1) * p.OW < nvalid && q * 4 < width) {
-                    const uint32_t box = sb + (q >> 3) * sbox_bytes;
-                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                    for (int tap = 0; tap < 4; tap++) {   // the reference's order: (0,0), (0,1), (1,0), (1,1)
-                        const int mm = (2 * prow + (tap >> 1)) * p.OW + 2 * pcol + (tap & 1);
-                        const float4 t = lds128f(box + mm * 128 + (((q & 7) ^ (mm & 7)) << 4));
-                        acc.x = __fadd_rn(acc.x, t.x); acc.y = __fadd_rn(acc.y, t.y); acc.z = __fadd_rn(acc.z, t.z); acc.w = __fadd_rn(acc.w, t.w);
-                    }
-                    const size_t e = ((((size_t)img0 * (p.OH >> 1) + (oh0 >> 1) + prow) * pw) + pcol) * p.N + n0 + cb + q * 4;
-                    *reinterpret_cast<float4*>(p.pool_out + e) =
-                        make_float4(__fdiv_rn(acc.x, 4.f), __fdiv_rn(acc.y, 4.f), __fdiv_rn(acc.z, 4.f), __fdiv_rn(acc.w, 4.f));
-                }
-                asm volatile("bar.sync 1, %0;" ::"n"(U8_EPILOGUE) : "memory");   // the tile has been read: it may be given back
-            }
-            if (et == 0) {
-                if (p.out)
-                    for (int hb = 0; hb < (width > 32 ? 2 : 1); hb++)
-                        asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
-                                     ::"l"(reinterpret_cast<uint64_t>(&out_map)), "r"(n0 + cb + hb * 32), "r"(oh0 * p.OW), "r"(img0),
-                                       "r"(sb + hb * sbox_bytes) : "memory");
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            }
-            if (++st_idx == p.stiles) { st_idx = 0; sc_par ^= 1u; }
-            if (++blk == nblk) {
-                blk = 0;
-                tile = next_tile(tile, ti++);
-                if (++accbuf == U8_ACCS) { accbuf = 0; accuse++; }
+                for (int s = 0; s < 4; s++) e.fetch(s, at, limit, p.narrow);
             }
         }
-        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        // POOL: the group folds its item's 32 channels: a thread takes four of them (pool_quad) of the tile's pooled pixels
+        // pool_px, pool_px + 16, ...
+        const int tid_g = (ew & 3) * 32 + lane, pool_quad = tid_g & 7, pool_px = tid_g >> 3, pw = p.OW >> 1, pool_pixels = (p.rows >> 1) * pw;
+        auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
+        bool alive = true;
+        while (alive && tile < p.ntiles) {
+            const int ptile = tile, pchunk = chunk;
+            {
+                // the item after this one, for the shortcut's prefetch
+                int k2 = k, chunk2 = chunk + EPI_GROUPS;
+                while (chunk2 >= nchunk) { chunk2 -= nchunk; k2++; }
+                const int tile2 = tile_of(k2);
+                long long base2 = 0;
+                int nvalid2 = 0;
+                const bool more = tile2 < p.ntiles;
+                if (more) tile_span(tile2, base2, nvalid2);
+                const int accbuf = k % U8_ACCS, cl = chunk * 32 + e.q * 8;
+                    alive = __all_sync(0xffffffffu, mbar_wait<64>(&bar_acc_full[accbuf], (k / U8_ACCS) & 1, abort_flag));
+                if (!alive) {
+                    atomicCAS(&g_u8_status, 0, 24);
+                    s_abort = 1;
+                    epi_abort = 1;
+                } else {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    e.take(tmem_base + ((uint32_t)r0 << 16) + accbuf * acc_cols + chunk * 32);
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bar_acc_empty[accbuf]);   // this warp's share of the accumulator has been read
+                    if (p.shortcut)
+                        e.finish<true, POOL>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), p.shortcut + element(base2, chunk2), more ? limit_of(nvalid2, chunk2) : 0u);
+                    else
+                        e.finish<false, POOL>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), nullptr, 0u);
+                }
+                k = k2; chunk = chunk2; tile = tile2; base = base2; nvalid = nvalid2;
+            }
+            if (POOL) {
+                // 2x2 average pooling of the item
+                group_sync();
+                if (epi_abort) break;
+                if (pchunk * 32 + pool_quad * 4 < n_this) {
+                    const int img = per_img(ptile), oh0 = (ptile - img * p.tiles_per_img) * p.rows;
+                    for (int pp = pool_px; pp < pool_pixels; pp += 16) {
+                        const int prow = pp / pw, pcol = pp - prow * pw;
+                        if (oh0 + 2 * prow + 1 >= p.OH) break;
+                        float4 x[4];
+#pragma unroll
+                        for (int tap = 0; tap < 4; tap++) {
+                            const int r = (2 * prow + (tap >> 1)) * p.P + 2 * pcol + (tap & 1);   // the accumulator row: its warp is the one
+                            const int w = group * 4 + ((r / 32 + 1) & 3);                         // whose index modulo four is r / 32
+                            x[tap] = lds128f(epi_addr + w * EPI_WARP_BYTES + (r & 31) * 128 + ((pool_quad ^ (r & 7)) << 4));
+                        }
+                        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                        for (int tap = 0; tap < 4; tap++) {   // the reference's order: (0,0), (0,1), (1,0), (1,1)
+                            acc.x = __fadd_rn(acc.x, x[tap].x); acc.y = __fadd_rn(acc.y, x[tap].y); acc.z = __fadd_rn(acc.z, x[tap].z); acc.w = __fadd_rn(acc.w, x[tap].w);
+                        }
+                        // (a quarter is a power of two: the product is the quotient)
+                        const size_t d = ((((size_t)img * (p.OH >> 1) + (oh0 >> 1) + prow) * pw) + pcol) * p.N + n0 + pchunk * 32 + pool_quad * 4;
+                        *reinterpret_cast<float4*>(p.pool_out + d) =
+                            make_float4(__fmul_rn(acc.x, 0.25f), __fmul_rn(acc.y, 0.25f), __fmul_rn(acc.z, 0.25f), __fmul_rn(acc.w, 0.25f));
+                    }
+                }
+                group_sync();   // the buffers may be overwritten
+            }
+        }
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

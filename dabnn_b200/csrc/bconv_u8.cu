@@ -10,7 +10,7 @@ namespace {
 
 struct U8Plan {
     int OH = 0, OW = 0, rows = 0, imgs = 0, tiles_per_img = 0, ntiles = 0, G = 0, stages = 0, wb = 0, nboxes = 0;
-    int smem = 0, resident = 0, stiles = 2, wide = 0, pair = 0, nbc = TC5_MAX_N, lag = 0;
+    int smem = 0, resident = 0, wide = 0, pair = 0, nbc = TC5_MAX_N;
 };
 
 // Shapes the engine takes: whole 64-channel groups, channel counts in 16s, stride 1 or 2 (even H and W), no
@@ -47,11 +47,7 @@ bool u8_plan(int n, int h, int w, int cin, int cout, int kh, int kw, int pad_h, 
     if (pl.wide) pl.G = 2;
     const int res_bytes = pl.nboxes * pl.wb * 64;
     pl.resident = res_bytes <= 48 * 1024;   // a channel block's weights stay in shared memory
-    // with resident weights the ring carries pixel boxes only and there is room for a third staging tile
-    pl.stiles = pl.resident ? 4 : 3;   // one more than the look-ahead needs: the latest tensor store may still be reading its tile
-    pl.lag = 1;
-    const int stile_bytes = u8_staging_tile_bytes(pl.rows * pl.OW * pl.imgs);
-    int avail = U8_MAX_SMEM - 1024 - pl.stiles * stile_bytes - 3072 /* static shared memory */;
+    int avail = U8_MAX_SMEM - 1024 - EPI_SMEM_BYTES - 3072 /* static shared memory */;
     if (pl.resident) avail -= res_bytes;
     // Streamed weights: two pixel tiles per weight stage (a stage is then two boxes of each tile and of the weights),
     // where handing out tiles in pairs does not lengthen the longest CTA's share (a few per cent per tile; a whole
@@ -71,7 +67,7 @@ bool u8_plan(int n, int h, int w, int cin, int cout, int kh, int kw, int pad_h, 
     const int stage_bytes = pl.G * ((pl.pair ? 2 : 1) * U8_BOX_BYTES + (pl.resident ? 0 : pl.wb * 64));
     pl.stages = std::min(8, avail / stage_bytes);
     if (pl.stages < 2) return false;
-    pl.smem = (pl.resident ? res_bytes : 0) + pl.stages * stage_bytes + pl.stiles * stile_bytes + 1024;
+    pl.smem = (pl.resident ? res_bytes : 0) + pl.stages * stage_bytes + EPI_SMEM_BYTES + 1024;
     return true;
 }
 
@@ -97,14 +93,12 @@ bool u8_input_maps(const unsigned char* in, int n, int h, int w, int cin, int st
 // ---- the halo kernel (bconv_halo.cuh): 3x3, stride 1, padding 1 --------------------------------------------------
 struct HaloPlan {
     int OH = 0, OW = 0, P = 0, rows = 0, tiles_per_img = 0, ntiles = 0, hslots = 0, halo_stride = 0, wstages = 0, wb = 0;
-    int resident = 0, stiles = 2, pair = 0, smem = 0;
-    int lag = 0;                   // see HaloParams
+    int resident = 0, pair = 0, smem = 0;
     int imgs = 1, img_pitch = 0;   // two whole images per tile (small images): accumulator rows between them
     int nb = TC5_MAX_N;            // output channels per CTA
 };
 
 int g_halo_mode = 1;   // 0: never, 1: wherever the shape allows (dabnn_debug_set_halo)
-int g_halo_stiles = 0; // 0: the plan's choice, else the number of staging tiles to try (dabnn_debug_set_halo, bits 4..7)
 
 // even_rows: tiles of an even number of output rows (the block also writes its 2x2 average pooling)
 bool halo_plan(int n, int h, int w, int cin, int cout, int kh, int kw, int pad_h, int pad_w, int stride_h, int stride_w,
@@ -127,7 +121,7 @@ bool halo_plan(int n, int h, int w, int cin, int cout, int kh, int kw, int pad_h
         int rmax = 128 / pl.P;
         if (even_rows) {
             rmax &= ~1;
-            if (rmax < 2 || (h & 1) || (w & 1) || (rmax / 2) * (w / 2) * 16 > U8_EPILOGUE) return false;
+            if (rmax < 2 || (h & 1) || (w & 1)) return false;
         }
         pl.tiles_per_img = (h + rmax - 1) / rmax;
         pl.rows = (h + pl.tiles_per_img - 1) / pl.tiles_per_img;
@@ -140,15 +134,8 @@ bool halo_plan(int n, int h, int w, int cin, int cout, int kh, int kw, int pad_h
     pl.wb = u8_weight_rows(cout);
     const int wbox = pl.wb * 64, res_bytes = 9 * cw * wbox;
     pl.resident = res_bytes <= 48 * 1024;
-    // One staging tile more than the shortcut's look-ahead needs, so that the tensor store of the block just finished may
-    // still be reading its tile when the next shortcut is fetched (measured: 56x56 390 -> 374 us, 28x28 226 -> 216 us at
-    // batch 1024; a deeper look-ahead bought nothing).
-    pl.stiles = pl.resident ? 4 : 3;
-    pl.lag = 1;
-    if (g_halo_stiles) { pl.stiles = std::min(g_halo_stiles & 7, U8_MAX_STILES); pl.lag = (g_halo_stiles >> 3) & 1; }
     pl.halo_stride = (((pl.img_pitch + (pl.rows + 2) * pl.P + (two ? 1 : 0)) * 64) + 1023) & ~1023;
-    const int stile_bytes = u8_staging_tile_bytes(pl.imgs * pl.rows * pl.OW);
-    int avail = U8_MAX_SMEM - 1024 - pl.stiles * stile_bytes - 3072 /* static shared memory */;
+    int avail = U8_MAX_SMEM - 1024 - EPI_SMEM_BYTES - 3072 /* static shared memory */;
     {
         const int ctas = std::max(1, sm_count() / ((cout + TC5_MAX_N - 1) / TC5_MAX_N));
         const int units = (pl.ntiles + 1) / 2;
@@ -175,7 +162,7 @@ bool halo_plan(int n, int h, int w, int cin, int cout, int kh, int kw, int pad_h
     }
     pl.hslots = std::min(HL_MAX_HSLOTS, avail / pl.halo_stride);
     if (pl.hslots < 2 * np) return false;
-    pl.smem = 1024 + pl.hslots * pl.halo_stride + (pl.resident ? res_bytes : pl.wstages * 3 * wboxs) + pl.stiles * stile_bytes;
+    pl.smem = 1024 + pl.hslots * pl.halo_stride + (pl.resident ? res_bytes : pl.wstages * 3 * wboxs) + EPI_SMEM_BYTES;
     return true;
 }
 
@@ -244,69 +231,53 @@ int bconv_u8_block_impl(const unsigned char* in_u8, const unsigned char* w_img, 
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     DABNN_REQUIRE(al16(in_u8) && al16(w_img) && al16(shortcut) && al16(out_f32) && al16(out_u8) && al16(out_bits), DABNN_ERR_ARG,
                   "bconv_u8: pointers must be 16-byte aligned");
+    const int narrow = ((reinterpret_cast<uintptr_t>(shortcut) | reinterpret_cast<uintptr_t>(out_f32)) & 31) != 0;
     static thread_local int configured_device = -1;
     int dev = 0;
     DABNN_CUDA_OK(cudaGetDevice(&dev));
     if (configured_device != dev) {
         DABNN_CUDA_OK(cudaFuncSetAttribute(bconv_u8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, U8_MAX_SMEM - 3072));
         DABNN_CUDA_OK(cudaFuncSetAttribute(bconv_u8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, U8_MAX_SMEM - 3072));
-        DABNN_CUDA_OK(cudaFuncSetAttribute(bconv_halo_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, U8_MAX_SMEM - 3072));
-        DABNN_CUDA_OK(cudaFuncSetAttribute(bconv_halo_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, U8_MAX_SMEM - 3072));
+        for (auto kern : {bconv_halo_kernel<false, false>, bconv_halo_kernel<false, true>, bconv_halo_kernel<true, false>, bconv_halo_kernel<true, true>})
+            DABNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, U8_MAX_SMEM - 3072));
         configured_device = dev;
     }
     HaloPlan hp;
     DABNN_REQUIRE(!pool_out || (al16(pool_out) && halo_plan(n, h, w, cin, cout, kh, kw, pad_h, pad_w, stride_h, stride_w, hp, -1, true)), DABNN_ERR_SHAPE,
                   "bconv_u8: the pooled output needs a 3x3 stride-1 block with even height and width that the halo kernel takes");
     if (halo_plan(n, h, w, cin, cout, kh, kw, pad_h, pad_w, stride_h, stride_w, hp, -1, pool_out != nullptr)) {   // 3x3 stride 1: every input byte enters the SM once per tile
-        CUtensorMap in_map, out_map{}, sc_map{};
+        CUtensorMap in_map;
         DABNN_REQUIRE(halo_input_map(in_u8, n, h, w, cin, hp, &in_map), DABNN_ERR_CUDA, "bconv_u8: cannot encode the halo's tensor map");
-        {
-            const unsigned long long dims[3] = {(unsigned long long)cout, (unsigned long long)hp.OH * hp.OW, (unsigned long long)n};
-            const unsigned long long strides[2] = {(unsigned long long)cout * 4, (unsigned long long)cout * 4 * hp.OH * hp.OW};
-            const unsigned box[3] = {32u, (unsigned)(hp.rows * hp.OW), (unsigned)hp.imgs};
-            DABNN_REQUIRE(!out_f32 || make_f32_tensor_map(&out_map, out_f32, 3, dims, strides, box), DABNN_ERR_CUDA,
-                          "bconv_u8: cannot encode the output's tensor map");
-            DABNN_REQUIRE(!shortcut || make_f32_tensor_map(&sc_map, const_cast<float*>(shortcut), 3, dims, strides, box), DABNN_ERR_CUDA,
-                          "bconv_u8: cannot encode the shortcut's tensor map");
-        }
         HaloParams q{};
         q.w_img = w_img; q.a = a; q.b = b; q.shortcut = shortcut; q.out = out_f32; q.out_u8 = out_u8; q.out_bits = out_bits;
         q.pool_out = pool_out;
         q.B = n; q.OH = hp.OH; q.OW = hp.OW; q.N = cout; q.cw = cin / 64; q.P = hp.P; q.imgs = hp.imgs; q.img_pitch = hp.img_pitch; q.nb = hp.nb;
         q.rows = hp.rows; q.tiles_per_img = hp.tiles_per_img; q.ntiles = hp.ntiles;
         q.hslots = hp.hslots; q.halo_stride = hp.halo_stride; q.wstages = hp.wstages; q.wb = hp.wb;
-        q.resident = hp.resident; q.stiles = hp.stiles; q.pair = hp.pair; q.lag = hp.lag;
+        q.resident = hp.resident; q.pair = hp.pair; q.narrow = narrow;
         const int tiles_n = (cout + hp.nb - 1) / hp.nb;
         const int per_n = std::max(1, sm_count() / tiles_n);
         const int nunits = hp.pair ? (hp.ntiles + 1) / 2 : hp.ntiles;
         dim3 grid(std::min(nunits, per_n), tiles_n);
-        if (hp.pair) launch_overlapped(bconv_halo_kernel<true>, grid, HL_THREADS, hp.smem, stream, q, in_map, out_map, sc_map);
-        else launch_overlapped(bconv_halo_kernel<false>, grid, HL_THREADS, hp.smem, stream, q, in_map, out_map, sc_map);
+        auto kern = hp.pair ? (pool_out ? bconv_halo_kernel<true, true> : bconv_halo_kernel<true, false>)
+                            : (pool_out ? bconv_halo_kernel<false, true> : bconv_halo_kernel<false, false>);
+        launch_overlapped(kern, grid, HL_THREADS, hp.smem, stream, q, in_map);
         return check_launch("bconv_halo_kernel");
     }
-    CUtensorMap in_maps[2], out_map{}, sc_map{};
+    CUtensorMap in_maps[2];
     DABNN_REQUIRE(u8_input_maps(in_u8, n, h, w, cin, stride_h, pl, in_maps), DABNN_ERR_CUDA, "bconv_u8: cannot encode the input's tensor map");
-    {
-        const unsigned long long dims[3] = {(unsigned long long)cout, (unsigned long long)pl.OH * pl.OW, (unsigned long long)n};
-        const unsigned long long strides[2] = {(unsigned long long)cout * 4, (unsigned long long)cout * 4 * pl.OH * pl.OW};
-        const unsigned box[3] = {32u, (unsigned)(pl.rows * pl.OW), (unsigned)pl.imgs};
-        DABNN_REQUIRE(!out_f32 || make_f32_tensor_map(&out_map, out_f32, 3, dims, strides, box), DABNN_ERR_CUDA,
-                      "bconv_u8: cannot encode the output's tensor map");
-        DABNN_REQUIRE(!shortcut || make_f32_tensor_map(&sc_map, const_cast<float*>(shortcut), 3, dims, strides, box), DABNN_ERR_CUDA,
-                      "bconv_u8: cannot encode the shortcut's tensor map");
-    }
     U8Params p{};
     p.w_img = w_img; p.a = a; p.b = b; p.shortcut = shortcut; p.out = out_f32; p.out_u8 = out_u8; p.out_bits = out_bits;
     p.B = n; p.OH = pl.OH; p.OW = pl.OW; p.N = cout;
     p.kh = kh; p.kw = kw; p.pad_h = pad_h; p.pad_w = pad_w; p.stride = stride_h; p.cw = cin / 64;
     p.rows = pl.rows; p.imgs = pl.imgs; p.tiles_per_img = pl.tiles_per_img; p.ntiles = pl.ntiles;
-    p.G = pl.G; p.stages = pl.stages; p.wb = pl.wb; p.nboxes = pl.nboxes; p.resident = pl.resident; p.stiles = pl.stiles; p.wide = pl.wide; p.pair = pl.pair; p.nbc = pl.nbc; p.lag = pl.lag;
+    p.G = pl.G; p.stages = pl.stages; p.wb = pl.wb; p.nboxes = pl.nboxes; p.resident = pl.resident; p.wide = pl.wide; p.pair = pl.pair; p.nbc = pl.nbc; p.narrow = narrow;
     const int tiles_n = (cout + pl.nbc - 1) / pl.nbc;
     const int per_n = std::max(1, sm_count() / tiles_n);
     const int nunits = pl.pair ? (pl.ntiles + 1) / 2 : pl.ntiles;
     dim3 grid(std::min(nunits, per_n), tiles_n);
-    if (pl.pair) launch_overlapped(bconv_u8_kernel<true>, grid, U8_THREADS, pl.smem, stream, p, in_maps[0], in_maps[1], out_map, sc_map);
-    else launch_overlapped(bconv_u8_kernel<false>, grid, U8_THREADS, pl.smem, stream, p, in_maps[0], in_maps[1], out_map, sc_map);
+    if (pl.pair) launch_overlapped(bconv_u8_kernel<true>, grid, U8_THREADS, pl.smem, stream, p, in_maps[0], in_maps[1]);
+    else launch_overlapped(bconv_u8_kernel<false>, grid, U8_THREADS, pl.smem, stream, p, in_maps[0], in_maps[1]);
     return check_launch("bconv_u8_kernel");
 }
 
@@ -326,7 +297,6 @@ using namespace dabnn;
 
 extern "C" int dabnn_debug_set_halo(int mode) {
     g_halo_mode = (mode & 15) != 0;
-    g_halo_stiles = (mode >> 4) & 15;
     return DABNN_OK;
 }
 

@@ -64,6 +64,16 @@ inline int conv_out_dim(int in, int pad, int dil, int k, int stride) {
     return (in + 2 * pad - (dil * (k - 1) + 1)) / stride + 1;
 }
 
+// The warp's index as a value the compiler knows to be the same in all its lanes: control flow and arithmetic that depend on
+// it stay on the uniform datapath.  A role whose every lane walks the loop, with only the asynchronous instruction itself
+// behind elect_lane(), hands the tensor core descriptors in uniform registers; behind `if (lane == 0)` each of them costs
+// moves from vector registers that take longer than the MMA.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_lane() {   // true in one lane of a converged warp
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

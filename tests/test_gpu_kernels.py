@@ -377,6 +377,31 @@ def test_float_layers_golden(ops, k):
                                k["ref_fconv_p0_s1"], rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("n,h,w,cin,cout,stride,pooled", [
+    (3, 14, 14, 64, 64, 1, False), (2, 28, 28, 64, 96, 1, True),   # the halo kernel: half a channel block, pooling of three items
+    (5, 7, 7, 128, 48, 1, False), (3, 16, 16, 64, 144, 2, False),  # two images per tile, an item of 16 channels; the per-tap kernel
+])
+def test_bconv_u8_block_shortcut_on_a_16_byte_boundary(ops, n, h, w, cin, cout, stride, pooled):
+    """The epilogue moves 32 bytes per lane where shortcut and output allow it and 16 otherwise: the same bits either way."""
+    g = torch.Generator(device="cuda").manual_seed(h + cout)
+    x8 = torch.randint(0, 2, (n, h, w, cin), device="cuda", dtype=torch.uint8, generator=g)
+    wt = torch.randint(-2**63, 2**63 - 1, (cout * 9 * cin // 64,), device="cuda", dtype=torch.int64, generator=g)
+    we = ops.bconv_u8_expand_weights(wt, cout, 9 * cin // 64)
+    a, b = torch.randn(cout, device="cuda", generator=g), torch.randn(cout, device="cuda", generator=g)
+    oh, ow = (h - 1) // stride + 1, (w - 1) // stride + 1
+    room = torch.randn(n * oh * ow * cout + 8, device="cuda", generator=g)
+    room = room[(-(room.data_ptr() // 4)) % 8:]                     # starts on a 32-byte boundary
+    shifted = room[4:4 + n * oh * ow * cout].view(n, oh, ow, cout)   # and this one does not
+    assert shifted.data_ptr() % 32 == 16
+    block = ops.bconv_u8_block_pooled if pooled else ops.bconv_u8_block
+    got = [block(x8, we, cout, 3, 3, 1, 1, stride, stride, a, b, sc, want_u8=True) for sc in (shifted, shifted.clone())]
+    for x, y in zip(*got):
+        assert x is None or torch.equal(x, y)
+    if pooled:
+        assert torch.equal(got[0][2], ops.avepool(got[0][0], 2, 2, 0, 0, 2, 2))
+    assert ops.engine_status() == 0
+
+
 @pytest.mark.parametrize("shape", [(2, 56, 56, 64), (3, 7, 7, 512), (2, 5, 3, 7), (1, 1, 1, 1000), (2, 9, 11, 64), (1, 18, 6, 128)])
 def test_float_layers_random(ops, port, shape):
     rng = np.random.default_rng(sum(shape))
