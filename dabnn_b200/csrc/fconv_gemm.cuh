@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_abort, epi_abort;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     unsigned char* stage0 = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
     unsigned char* stile = stage0 + stages * FG_STAGE_BYTES;
     const volatile int* abort_flag = &s_abort;
@@ -174,8 +174,9 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                 if (++s == (uint32_t)stages) { s = 0; par ^= 1u; }
             }
     } else if (warp == FG_MMA_WARP) {
-        // =========================== MMA issue: one lane ===========================
-        if (lane == 0) {
+        // =========================== MMA issue: the whole warp walks, one lane issues ===========================
+        {
+            const bool leader = elect_lane();
             const uint32_t idesc_m = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(128 >> 4) << 24);   // D f32, A = B = tf32, K-major, M = 128
             const uint64_t d_stage = fg_desc_sw128(smem_u32(stage0));
             constexpr uint32_t TILE_UNITS = FG_TILE_BYTES >> 4, STAGE_UNITS = FG_STAGE_BYTES >> 4;
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
             int i = 0;
             for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, i++) {
                 const int accbuf = i % FG_ACCS, accuse = i / FG_ACCS;
-                if (accuse >= 1 && !mbar_wait(&bar_acc_empty[accbuf], (accuse - 1) & 1, abort_flag)) {
+                if (accuse >= 1 && !mbar_wait_warp(&bar_acc_empty[accbuf], (accuse - 1) & 1, abort_flag)) {
                     atomicCAS(&g_tc5_status, 0, 43);
                     s_abort = 1;
                     break;
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                 uint32_t accum = 0;
                 int cg = 0;
                 for (int c = 0; c < nchunks; c++) {
-                    if (!mbar_wait(&bar_ready[s], par, abort_flag)) {
+                    if (!mbar_wait_warp(&bar_ready[s], par, abort_flag)) {
                         atomicCAS(&g_tc5_status, 0, 44);
                         s_abort = 1;
                         ok = false;
@@ -215,18 +216,21 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                         }
                     };
                     const int left = p.cin - cg * FG_CHUNK;
+                    if (leader) {
                     if (left >= FG_CHUNK) {
 #pragma unroll
                         for (int j = 0; j < FG_CHUNK / 8; j++) slice(j);
                     } else {   // the last channel group of a tap: only the slices that hold channels
                         for (int j = 0; j * 8 < left; j++) slice(j);
                     }
+                    umma_commit(&bar_empty[s]);
+                    }
                     if (++cg == cgroups) cg = 0;
                     accum = 1u;
-                    umma_commit(&bar_empty[s]);
                     if (++s == (uint32_t)stages) { s = 0; par ^= 1u; }
                 }
-                if (ok) umma_commit(&bar_acc_full[accbuf]);
+                if (ok && leader) umma_commit(&bar_acc_full[accbuf]);
+                __syncwarp();
             }
         }
     } else {

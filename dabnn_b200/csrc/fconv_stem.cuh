@@ -33,12 +33,16 @@
 //   * 16 epilogue warps, thread (pixel, 16-channel quarter), in two groups of eight, one per 32-channel box:
 //     tcgen05.ld, add the two column halves, bias, affine, relu, park the row in the group's 128-byte-swizzled
 //     staging box, one TMA tensor store per box.
+// What bounds it: the shared-memory pipe (2.5 k of about 3.4 k cycles per output row are the MMA's operand reads).  On
+// 1024 images of 224x224 the issuing thread alone behind `if (lane == 0)`, and affine + relu on every value, took 1590 us;
+// a warp-uniform issue loop and affine + relu on the pooled values only, 1342 us.
 // With POOL the 3x3 stride-2 pad-1 max pooling that follows a ResNet stem happens in the same kernel and the stem's own
 // output never leaves the SM: a CTA's share is a run of POOLED rows, the stem rows under them arrive in order (the
 // first one computed again by the neighbour that shares it).  An epilogue thread meets the same pixel column in every
 // row, so it folds the window's rows in registers with the reference's `acc < t ? t : acc` rule; every second stem row
 // completes a pooled row, which alone is parked in the staging boxes, folded over its three columns and written out as
-// fp32 and as {0,1} sign bytes.  The values are those of the two layers run one after the other (the maximum does not
+// fp32 and as {0,1} sign bytes.  Affine and relu are applied to the completed maxima only (both are monotone per channel:
+// the sums are folded with their sign flipped where the affine's factor is negative).  The values are those of the two layers run one after the other (the maximum does not
 // depend on the order of the fold; the only freedom is which zero comes out of a window whose maximum is both +0 and
 // -0, where the reference's tap order is row-major and this one is column-major).
 // Every wait is bounded; a wait that gives up records a code (31 converters, 32 / 33 MMA thread waiting for rows /
@@ -84,6 +88,18 @@ __device__ __forceinline__ float4 fs_sel(const float4 a, const float4 t) {
     return make_float4(a.x < t.x ? t.x : a.x, a.y < t.y ? t.y : a.y, a.z < t.z ? t.z : a.z, a.w < t.w ? t.w : a.w);
 }
 
+// affine (a: the factor's magnitude; its sign is in the value already) and relu of a pooled value
+__device__ __forceinline__ float4 fs_finish(float4 h, const float4 a, const float4 b, bool affine, int relu) {
+    float v[4] = {h.x, h.y, h.z, h.w};
+    const float ka[4] = {a.x, a.y, a.z, a.w}, kb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        if (affine) v[e] = __fadd_rn(__fmul_rn(ka[e], v[e]), kb[e]);
+        if (relu) v[e] = relu_ref(v[e]);
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
+}
+
 // K-major SWIZZLE_32B shared-memory descriptor: rows of 32 bytes, 8-row groups 256 bytes apart
 __device__ __forceinline__ uint64_t umma_desc_sw32(uint32_t saddr) {
     return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(256 >> 4) << 32) | ((uint64_t)1 << 46) |
@@ -127,8 +143,9 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_abort, epi_abort[2];
     __shared__ __align__(16) float chan_bias[FS_N], chan_a[FS_N], chan_b[FS_N];
+    __shared__ __align__(16) uint32_t chan_flip[FS_N];   // POOL: the sign bit where the affine's factor is negative
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int n0 = blockIdx.y * FS_N;
     const int n_this = min(FS_N, p.cout - n0);                  // multiple of 16 (host-checked)
     unsigned char* patch = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
@@ -176,6 +193,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
         chan_bias[tid] = (in && p.bias) ? __ldg(p.bias + n0 + tid) : 0.f;
         chan_a[tid] = (in && p.a) ? __ldg(p.a + n0 + tid) : 1.f;
         chan_b[tid] = (in && p.a) ? __ldg(p.b + n0 + tid) : 0.f;
+        chan_flip[tid] = __float_as_uint(chan_a[tid]) & 0x80000000u;
+        if (POOL) chan_a[tid] = fabsf(chan_a[tid]);
     }
     // resident weights, K order (ky, kx < kxp, c < 4): element (n, k) -> (n / 8) * w_sbo + (k / 4) * 128 + (n % 8) * 16 + (k % 4) * 4
     // (four elements per thread and step, their loads issued together: the set-up is a fixed cost of every launch)
@@ -314,8 +333,9 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
             }
         }
     } else if (warp == FS_MMA_WARP) {
-        // =========================== MMA issue: one lane ===========================
-        if (lane == 0) {
+        // =========================== MMA issue: the whole warp walks, one lane issues ===========================
+        {
+            const bool leader = elect_lane();
             const uint32_t idesc_m = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(128 >> 4) << 24);   // D f32, A = B = tf32, K-major, M = 128
             const uint32_t idesc = idesc_m | ((uint32_t)(n_this >> 3) << 17);
             const bool stacked = n_this == FS_N;
@@ -329,19 +349,19 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
             constexpr int SLICES2 = (SLICES + 1) / 2;
             const uint64_t d_wh = umma_desc_kmajor(smem_u32(wbase), 128, w_sbo), d_wl = umma_desc_kmajor(smem_u32(wbase) + w_half, 128, w_sbo);
             const uint32_t slot_units = (uint32_t)g.slot_bytes >> 4;
-            // The issuing thread is one instruction stream and an MMA of this size executes in 50 - 65 cycles: the loop
+            // The issuing warp is one instruction stream and an MMA of this size executes in 50 - 65 cycles: the loop
             // must cost less than that per instruction, so the slices of a window row are unrolled (descriptors advance
             // by constants) and the two forms of the hi product get their own loops.
             FsTileIter it;
             it.init(g_begin, p.oh);
             for (; it.t < ntiles; it.advance(p.oh, p.kh, p.stride_h, g.slots)) {
                 const int t = it.t, accbuf = t % FS_ACCS, accuse = t / FS_ACCS;
-                if (accuse >= 1 && !mbar_wait(&acc_empty[accbuf], (accuse - 1) & 1, abort_flag)) {
+                if (accuse >= 1 && !mbar_wait_warp(&acc_empty[accbuf], (accuse - 1) & 1, abort_flag)) {
                     atomicCAS(&g_tc5_status, 0, 33);
                     s_abort = 1;
                     break;
                 }
-                if (!mbar_wait(&rows_ready[t & 3], (t >> 2) & 1, abort_flag)) {   // the issuing thread is the critical path: no sleep between polls
+                if (!mbar_wait_warp(&rows_ready[t & 3], (t >> 2) & 1, abort_flag)) {   // the issuing thread is the critical path: no sleep between polls
                     atomicCAS(&g_tc5_status, 0, 32);
                     s_abort = 1;
                     break;
@@ -351,6 +371,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
                 uint64_t bh = d_wh, bl = d_wl, b2 = d_w2;
                 uint32_t accum = 0;
                 int slot = it.s0;
+                if (leader) {
                 // one slice = eight floats = two 16-byte units per row: 32 bytes of a window row, 256 bytes of the weight layout
                 if (stacked) {
                     for (int ky = 0; ky < p.kh; ky++) {
@@ -382,6 +403,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
                     }
                 }
                 umma_commit(&tile_done[accbuf]);   // the accumulator is complete and the window's slots have been read
+                }
+                __syncwarp();
             }
         }
     } else {
@@ -424,8 +447,24 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
                                  : "=r"(xx[0]), "=r"(xx[1]), "=r"(xx[2]), "=r"(xx[3]), "=r"(xx[4]), "=r"(xx[5]), "=r"(xx[6]), "=r"(xx[7])
                                  : "r"(t_addr + FS_N + half * 8));
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (POOL) {
+                        // Affine and relu are monotone per channel, so they wait for the window's maximum (a quarter of the
+                        // values): with the sign flipped where the affine's factor is negative, a maximum it is.
 #pragma unroll
-                    for (int q = 0; q < 2; q++) {   // the channel constants four at a time: every shared-memory wavefront counts here
+                        for (int q = 0; q < 2; q++) {
+                            const int cl = cq * 16 + half * 8 + q * 4;
+                            const uint4 fl = *reinterpret_cast<const uint4*>(chan_flip + cl);
+                            const uint32_t f4[4] = {fl.x, fl.y, fl.z, fl.w};
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                float f = __uint_as_float(y[q * 4 + e]) + __uint_as_float(xx[q * 4 + e]);   // + the hi*lo part
+                                if (p.bias) f = __fadd_rn(f, chan_bias[cl + e]);
+                                y[q * 4 + e] = __float_as_uint(f) ^ f4[e];
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < (POOL ? 0 : 2); q++) {   // the channel constants four at a time: every shared-memory wavefront counts here
                         const int cl = cq * 16 + half * 8 + q * 4;
                         const float4 cbias = *reinterpret_cast<const float4*>(chan_bias + cl), ca = *reinterpret_cast<const float4*>(chan_a + cl),
                                      cb = *reinterpret_cast<const float4*>(chan_b + cl);
@@ -457,7 +496,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
 #pragma unroll
                     for (int e = 0; e < 16; e++) {
                         const float f = __uint_as_float(v[e]);
-                        vmax[e] = init ? f : (vmax[e] < f ? f : vmax[e]);
+                        vmax[e] = init ? f : fmaxf(vmax[e], f);
                     }
                 }
                 if (!emit) continue;   // (a warp that gave up runs on, idle, to the next barrier and leaves with its group)
@@ -484,6 +523,9 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
                         const int ox = 2 * px + dx;
                         if ((unsigned)ox < (unsigned)p.ow) h = fs_sel(h, lds128f(sbox + ox * 128 + ((q ^ (ox & 7)) << 4)));
                     }
+                    // (a product of the flipped sum and the factor's magnitude is the product of the two themselves)
+                    h = fs_finish(h, *reinterpret_cast<const float4*>(chan_a + h2 * 32 + q * 4), *reinterpret_cast<const float4*>(chan_b + h2 * 32 + q * 4),
+                                  p.a != nullptr, p.relu);
                     const size_t e = (((size_t)img * g.ph + (oy >> 1)) * g.pw + px) * p.cout + n0 + h2 * 32 + q * 4;
                     *reinterpret_cast<float4*>(pool_out + e) = h;
                     if (pool_u8)
