@@ -463,9 +463,4 @@ __global__ void __launch_bounds__(WM* WN * 32, 2)
     cp_async_wait<0>();
 }
 
-// Host-side launcher: picks the tile shape from N and dispatches on the engine.
-template <class XOp, class WOp>
-int launch_bcontract(int engine, const XOp& xop, const WOp& wop, const EpilogueParams& ep, int M, int N,
-                     int kwords, cudaStream_t stream);
-
 }  // namespace dabnn

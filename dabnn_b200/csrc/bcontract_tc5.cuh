@@ -9,9 +9,9 @@
 // A CTA (one per SM, persistent over pixel tiles) works on 128-pixel x (up to) 128-channel tiles
 // with three kinds of warps that only meet at mbarriers:
 //   * 8 producer warps; thread (r, h) owns half of the 64-bit words of every K chunk of operand row
-//     r (chunks of 128 bits through four stages for short K, 256 bits through two stages otherwise:
-//     Tc5Cfg).  It reads its words (implicit im2col: tap by tap, zero word outside the image; the tap
-//     decode is stepped, not divided), expands every 32 bits to 32 bytes with shift+mask pairs
+//     r (chunks of 256 bits through two stages: Tc5Cfg).  It reads its words (implicit im2col: tap
+//     by tap, zero word outside the image; the tap decode is stepped, not divided), expands every
+//     32 bits to 32 bytes with shift+mask pairs
 //     ((w >> s) & 0x01010101 - the resulting bit -> K-slot permutation is the same for both
 //     operands, and a contraction is blind to it) and stores them in the K-major SWIZZLE_NONE
 //     canonical layout of UMMA shared-memory descriptors (8 rows x 16 B core matrices).  Loads run
@@ -96,14 +96,11 @@ __device__ __forceinline__ void mma_i8_ss(uint32_t d_tmem, uint64_t ad, uint64_t
                  ::"r"(d_tmem), "l"(ad), "l"(bd), "r"(idesc), "r"(accum), "r"(0), "r"(0), "r"(0), "r"(0) : "memory");
 }
 
-// Shapes that depend on the K chunk: CW 64-bit words per chunk (a producer thread owns CW / 2 of them) and
-// 8 / CW ring stages, 128 KB of stages either way.  Long chunks amortise the per-stage hand-shake (a
-// tcgen05.commit alone costs the issuing thread ~270 cycles) over more MMAs; short K keeps short chunks so
-// that its few words still spread over several stages.
-template <int CW>
+// 256 bits of K per chunk and two ring stages (128 KB): long chunks amortise the per-stage hand-shake (a tcgen05.commit alone
+// costs the issuing thread ~270 cycles) over more MMAs.
 struct Tc5Cfg {
-    static constexpr int WORDS = CW, WPT = CW / 2, STAGES = 8 / CW;
-    static constexpr int CHUNK_BYTES = CW * 64;                      // operand bytes per row per chunk
+    static constexpr int WORDS = 4, WPT = WORDS / 2, STAGES = 2;     // words per chunk, of which a producer thread owns WPT
+    static constexpr int CHUNK_BYTES = WORDS * 64;                    // operand bytes per row per chunk
     static constexpr int SBO = (CHUNK_BYTES / 16) * 128;             // byte stride between 8-row groups
     static constexpr int A_BYTES = 128 * CHUNK_BYTES;
     static constexpr int B_BYTES = TC5_MAX_N * CHUNK_BYTES;
@@ -115,7 +112,6 @@ struct Tc5Cfg {
     static constexpr int STILE_BYTES = 2 * SBOX_BYTES;               // 32 KB: 128 pixels x 64 channels of fp32
     static constexpr int TOTAL = STAGES * STAGE_BYTES + 2 * STILE_BYTES + 1024 /*alignment slack*/;
 };
-__host__ __device__ inline int tc5_chunk_words(int kwords) { return kwords <= 12 ? 2 : 4; }
 
 // 32 bits -> 32 bytes {0,1}: output word s holds bits s, s+8, s+16, s+24.  Two 16-byte stores.
 __device__ __forceinline__ void expand32(unsigned char* dst_unit0, uint32_t w) {
@@ -147,15 +143,14 @@ __device__ __forceinline__ void expand_word_smem(uint32_t dst, uint64_t w) {
 // become one bulk copy (global -> shared, completion on the stage's "full" mbarrier) issued by one thread.
 // The buffer ends with the popcount of every weight row (one int per channel, padded to whole channel blocks).
 __host__ __device__ inline size_t tc5_expanded_image_bytes(int N, int kwords) {
-    const int cw = tc5_chunk_words(kwords);
-    return (size_t)((N + TC5_MAX_N - 1) / TC5_MAX_N) * ((kwords + cw - 1) / cw) * (TC5_MAX_N * cw * 64);
+    return (size_t)((N + TC5_MAX_N - 1) / TC5_MAX_N) * ((kwords + Tc5Cfg::WORDS - 1) / Tc5Cfg::WORDS) * Tc5Cfg::B_BYTES;
 }
 __host__ __device__ inline size_t tc5_expanded_bytes(int N, int kwords) {
     return tc5_expanded_image_bytes(N, kwords) + (size_t)((N + TC5_MAX_N - 1) / TC5_MAX_N) * TC5_MAX_N * sizeof(int);
 }
-template <int CW, class WOp>
+template <class WOp>
 __global__ void __launch_bounds__(256) tc5_expand_weights_kernel(const WOp wop, const int N, const int kwords, unsigned char* dst) {
-    using C = Tc5Cfg<CW>;
+    using C = Tc5Cfg;
     const int c = blockIdx.x, nt = blockIdx.y, r = threadIdx.x & 127, h = threadIdx.x >> 7;
     const int n = nt * TC5_MAX_N + r;
     for (int j = 0; j < C::WPT; j++) {
@@ -182,11 +177,11 @@ __global__ void __launch_bounds__(256) tc5_expand_weights_kernel(const WOp wop, 
     }
 }
 
-template <int CW, class XOp, class WOp>
+template <class XOp, class WOp>
 __global__ void __launch_bounds__(TC5_THREADS, 1)
     bcontract_tc5_kernel(const XOp xop, const WOp wop, const EpilogueParams ep, const int M, const int N,
                          const int kwords, const int ntiles_m, const __grid_constant__ CUtensorMap out_map) {
-    using C = Tc5Cfg<CW>;
+    using C = Tc5Cfg;
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t bar_full[C::STAGES], bar_empty[C::STAGES], bar_acc_full[TC5_ACCS], bar_acc_empty[TC5_ACCS];
     __shared__ uint32_t tmem_base_s;

@@ -1,0 +1,318 @@
+// Binary contraction with the pixel operand in tensor memory: tcgen05.mma kind::i8, A from TMEM, B resident in shared memory.
+//
+//   cnt[p][n] = sum_k x[p][k] XOR w[n][k] = popc(w[n]) + sum_k x[p][k] * (1 - 2 w[n][k])
+//
+// with 1 - 2 w as +1 / -1 bytes.  The kernel of bcontract_tc5.cuh expands both operands into shared memory for every tile, and
+// its shared-memory pipe is what runs out: per 32 bytes of K it writes 8 KB and the tensor core reads them back.  Here
+//   * the CTA's filters are expanded once, before the first tile, and stay in shared memory (the channel block is narrowed
+//     until they fit: tmem_plan in contraction.cu);
+//   * the producers, thread = pixel row, write their expanded bytes with tcgen05.st straight to the tensor-memory columns that
+//     the MMA reads as its A operand (lane = row, a column = four bytes of K): no shared-memory traffic at all;
+//   * the +1 / -1 filters make the accumulator the count less popc(w): nothing per pixel row travels to the epilogue;
+//   * the epilogue is the one of independent warps (bconv_epilogue.cuh).
+// Both operands use the same bit -> K-slot permutation (expand32), which a contraction is blind to.
+//
+// What bounds it: the producers' instruction issue at long K, the epilogue (and HBM: the fp32 output and shortcut) at short K.
+// Against the kernel of bcontract_tc5.cuh, us a launch: block of 256 x 28x28x128 -> 128 3x3 with shortcut 78.5 -> 53.6 (206 MB,
+// 32 us at the copy rate), 256 x 56x56x64 -> 64 179 -> 98, 256 x 14x14x256 -> 256 72 -> 49; 256 x 14x14x256 -> 512 1x1 49 -> 27;
+// 802816 x 64 x 576 GEMM 150 -> 87; 49 x 512 x 4608 25 -> 10.5.  Left shifts instead of right ones in the expansion: 14x14x256
+// 54 -> 49, 7x7x512 at 32 channels 85 -> 75; groups of producers in turn instead of half a stage each: 72 -> 54.
+//
+// Tensor memory: columns 0 - 255 hold the accumulators, 256 - 511 four stages of 64 columns (256 bits of K).
+// Every wait on an mbarrier is bounded, with the status codes of bcontract_tc5.cuh.
+#pragma once
+#include "bconv_epilogue.cuh"
+
+namespace dabnn {
+
+constexpr int TM_STAGES = 4, TM_WORDS = 4;           // ring stages, 64-bit words of K per stage
+constexpr int TM_STAGE_COLS = TM_WORDS * 16, TM_A_COL = 256;
+constexpr int TM_AHEAD = 3;                          // stages of its own that a producer's loads run ahead
+constexpr int TM_WARPS = 16;                         // producers + epilogue
+constexpr int TM_THREADS = TM_WARPS * 32 + 32;
+constexpr int TM_MAX_ACCS = 4;
+constexpr int TM_MAX_LD = 1 << 24;                   // output pitch (the epilogue's 32-bit offsets within a tile)
+
+struct TmemPlan {
+    int nbc;                                         // channels per CTA
+    int producer_warps;                              // 4, 8 or 12
+};
+__host__ __device__ inline int tmem_smem_bytes(int nbc, int kwords, int producer_warps) {
+    return kwords * nbc * 64 + (TM_WARPS - producer_warps) * EPI_WARP_BYTES + 128 /*alignment slack*/;
+}
+
+__device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bd, uint32_t idesc, uint32_t accum) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}\n"
+                 ::"r"(d_tmem), "r"(a_tmem), "l"(bd), "r"(idesc), "r"(accum), "r"(0), "r"(0), "r"(0), "r"(0) : "memory");
+}
+// One 64-bit word of the warp's 32 rows -> 16 tensor-memory columns, K slots as expand32 orders them.  A set bit becomes the byte
+// 128: left shifts are multiplications and leave the logic pipe, which the masks alone keep busy.  The accumulator is scaled
+// back, exactly, in the epilogue.
+constexpr float TM_SCALE = 1.f / 128.f;
+constexpr int TM_MAX_WORDS = (1 << 21) / 128 / 64 - 1;   // |accumulator| stays below 2^21 (EpiWarp::finish)
+__device__ __forceinline__ void tmem_st_word(uint32_t t_addr, uint64_t word) {
+    const uint32_t M = 0x80808080u, l = (uint32_t)word, h = (uint32_t)(word >> 32);
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(t_addr), "r"((l << 7) & M), "r"((l << 6) & M), "r"((l << 5) & M), "r"((l << 4) & M), "r"((l << 3) & M), "r"((l << 2) & M),
+                   "r"((l << 1) & M), "r"(l & M), "r"((h << 7) & M), "r"((h << 6) & M), "r"((h << 5) & M), "r"((h << 4) & M), "r"((h << 3) & M),
+                   "r"((h << 2) & M), "r"((h << 1) & M), "r"(h & M)
+                 : "memory");
+}
+
+// PW producer warps, the other 16 - PW are the epilogue.  The output pitch ep.ld_out is also the shortcut's; sign bits are
+// written for ep.ld_out == N only (host-checked).
+template <int PW, class XOp, class WOp>
+__global__ void __launch_bounds__(TM_THREADS, 1)
+    bcontract_tmem_kernel(const XOp xop, const WOp wop, const EpilogueParams ep, const int M, const int N, const int kwords, const int ntiles_m,
+                          const int nbc, const int narrow, const int weights_first) {
+    constexpr int EW = TM_WARPS - PW, EGROUPS = EW / 4, PGROUPS = PW / 4;
+    extern __shared__ unsigned char smem_dyn[];
+    __shared__ __align__(8) uint64_t bar_full[TM_STAGES], bar_empty[TM_STAGES], bar_acc_full[TM_MAX_ACCS], bar_acc_empty[TM_MAX_ACCS];
+    __shared__ uint32_t tmem_base_s;
+    __shared__ int s_abort, popw[TC5_MAX_N];
+    __shared__ __align__(16) float pop[TC5_MAX_N];
+    __shared__ __align__(16) float chan_a[TC5_MAX_N];
+    __shared__ __align__(16) float chan_b[TC5_MAX_N];
+
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
+    const int n0 = blockIdx.y * nbc, n_this = min(nbc, N - n0);              // a multiple of 16 (host-checked)
+    const int nchunks = (kwords + TM_WORDS - 1) / TM_WORDS;
+    const int acc_cols = (n_this + 31) & ~31, naccs = acc_cols > 64 ? 2 : TM_MAX_ACCS;   // columns per accumulator: whole 32-column items
+    const uint32_t wimg = (smem_u32(smem_dyn) + 127) & ~127u, wbox = (uint32_t)nbc * 64u;   // filters: [word][row / 8][unit][row % 8][16 bytes]
+    const uint32_t epi_smem = wimg + (uint32_t)kwords * wbox;
+    const volatile int* abort_flag = &s_abort;
+
+    if (warp == TM_WARPS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_base_s)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    if (tid == 0) {
+        for (int i = 0; i < TM_STAGES; i++) { mbar_init(&bar_full[i], 4); mbar_init(&bar_empty[i], 1); }
+        for (int i = 0; i < TM_MAX_ACCS; i++) { mbar_init(&bar_acc_full[i], 1); mbar_init(&bar_acc_empty[i], 4 * ((n_this + 31) >> 5)); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::);
+        s_abort = 0;
+    }
+    if (tid < TC5_MAX_N) popw[tid] = 0;
+    // Filters that no kernel still running may be writing are read while that kernel drains (weights_first); otherwise after it.
+    if (!weights_first) grid_dependency_wait();
+    if (tid < TC5_MAX_N) {
+        const bool have = ep.a && tid < n_this;
+        chan_a[tid] = have ? __ldg(ep.a + n0 + tid) : 1.f;
+        chan_b[tid] = have ? __ldg(ep.b + n0 + tid) : 0.f;
+    }
+    __syncthreads();
+    {   // thread = channel (lanes) x word, eight loads in flight
+        const int nlog = 31 - __clz(nbc);                                    // nbc is a power of two
+        const int r = tid & (nbc - 1), per = TM_WARPS * 32 >> nlog;
+        if (tid < TM_WARPS * 32 && r < n_this) {
+            const RowCtx row = wop.make_row(n0 + r);
+            const uint32_t dst = wimg + (r >> 3) * 512 + (r & 7) * 16;
+            int pc = 0;
+            for (int q0 = tid >> nlog; q0 < kwords; q0 += per * 8) {
+                uint64_t w[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int q = q0 + j * per;
+                    w[j] = 0;
+                    if (q < kwords) w[j] = __ldg(wop.addr(row, wop.decode(q)));
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int q = q0 + j * per;
+                    if (q < kwords) {
+                        pc += __popcll(w[j]);
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {                        // 16-byte unit u: bits s + 8 i of the half word, s = 4 (u & 1) ..
+                            const uint32_t half = (uint32_t)(w[j] >> (u >= 2 ? 32 : 0)) >> (4 * (u & 1));
+                            auto sgn = [](uint32_t x) { const uint32_t m = x & 0x01010101u; return (m * 0xffu) | (m ^ 0x01010101u); };   // 0 -> +1, 1 -> -1
+                            sts128(dst + (uint32_t)q * wbox + u * TC5_LBO, sgn(half), sgn(half >> 1), sgn(half >> 2), sgn(half >> 3));
+                        }
+                    }
+                }
+            }
+            atomicAdd(&popw[r], pc);
+        }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads what was just written
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = tmem_base_s;
+    if (weights_first) grid_dependency_wait();   // activations (and what is added to) come next
+
+    if (warp < PW) {
+        // =========================== producers: thread = operand row ===========================
+        // The groups of four warps take the stages in turn, so that a group has several stages' time for the chain wait - write -
+        // wait for the writes - hand over.  Its loads run TM_AHEAD of its stages ahead and do not stop at tile boundaries: the
+        // cursor below walks (tile, stage).
+        const int group = warp >> 2, r = (warp & 3) * 32 + lane;
+        const uint32_t a_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + TM_A_COL;
+        const bool pair = xop.pairable();
+        struct Words { uint64_t w[TM_WORDS]; };
+        int ltile = blockIdx.x, lchunk = group;
+        while (lchunk >= nchunks) { lchunk -= nchunks; ltile += gridDim.x; }
+        RowCtx xr = xop.make_row(ltile * 128 + r);
+        typename XOp::Dec xd = xop.decode(lchunk * TM_WORDS);
+        auto load_next = [&](Words& v) {
+            const int q = lchunk * TM_WORDS;
+#pragma unroll
+            for (int j = 0; j < TM_WORDS; j += 2) {
+                v.w[j] = 0; v.w[j + 1] = 0;
+                if (ltile < ntiles_m && q + j < kwords) {
+                    const uint64_t* p = xop.addr(xr, xd);
+                    if (pair && q + j + 1 < kwords) {                       // two words of one tap on a 16-byte boundary
+                        if (p) {
+                            const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(p));
+                            v.w[j] = t.x; v.w[j + 1] = t.y;
+                        }
+                        xop.advance(xd, 2);
+                    } else {
+                        if (p) v.w[j] = __ldg(p);
+                        xop.advance(xd, 1);
+                        if (q + j + 1 < kwords) {
+                            p = xop.addr(xr, xd);
+                            if (p) v.w[j + 1] = __ldg(p);
+                        }
+                        xop.advance(xd, 1);
+                    }
+                }
+            }
+            lchunk += PGROUPS;
+            if (lchunk < nchunks) {
+                xop.advance(xd, (PGROUPS - 1) * TM_WORDS);
+            } else {
+                do { lchunk -= nchunks; ltile += gridDim.x; } while (lchunk >= nchunks);
+                xr = xop.make_row(ltile * 128 + r);
+                xd = xop.decode(lchunk * TM_WORDS);
+            }
+        };
+        Words v[TM_AHEAD];
+#pragma unroll
+        for (int j = 0; j < TM_AHEAD; j++) load_next(v[j]);
+        const int total = ((ntiles_m - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * nchunks;   // stages of this CTA
+        bool ok = true;
+        for (int i = group; i < total && ok;) {
+#pragma unroll
+            for (int j = 0; j < TM_AHEAD; j++, i += PGROUPS) {
+                if (i >= total || !ok) break;
+                const uint32_t s = i % TM_STAGES, use = i / TM_STAGES;
+                if (use >= 1) ok = mbar_wait_warp(&bar_empty[s], (use - 1) & 1, abort_flag);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");   // the MMAs that read this stage are complete
+#pragma unroll
+                for (int w = 0; w < TM_WORDS; w++) tmem_st_word(a_addr + s * TM_STAGE_COLS + w * 16, v[j].w[w]);   // (words beyond K: zeros that no MMA reads)
+                load_next(v[j]);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_full[s]);
+            }
+        }
+        if (!ok) {
+            atomicCAS(&g_tc5_status, 0, 1);
+            s_abort = 1;
+        }
+    } else if (warp == TM_WARPS) {
+        // =========================== MMA issue: the whole warp walks, one lane issues ===========================
+        // instruction descriptor: D = s32, A = u8, B = s8, both K-major, N = n_this, M = 128
+        const uint32_t idesc = (2u << 4) | (1u << 10) | ((uint32_t)(n_this >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint64_t d_b = umma_desc(wimg, 512);
+        const uint32_t wbox_units = wbox >> 4;
+        const bool leader = elect_lane();
+        uint32_t s = 0, par = 0;
+        bool ok = true;
+        int acc = 0, accpar = 0, first = 1;
+        for (int tile = blockIdx.x; tile < ntiles_m && ok; tile += gridDim.x) {
+            if (!first && !mbar_wait_warp(&bar_acc_empty[acc], accpar ^ 1, abort_flag)) {
+                atomicCAS(&g_tc5_status, 0, 3);
+                s_abort = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t d_tmem = tmem_base + acc * acc_cols;
+            uint64_t bd = d_b;
+            for (int c = 0; c < nchunks; c++, bd += TM_WORDS * wbox_units) {
+                if (!mbar_wait_warp(&bar_full[s], par, abort_flag)) {
+                    atomicCAS(&g_tc5_status, 0, 4);
+                    s_abort = 1;
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int words = min(TM_WORDS, kwords - c * TM_WORDS);
+                const uint32_t at = tmem_base + TM_A_COL + s * TM_STAGE_COLS;
+                if (leader) {   // one MMA per 32 bytes of K: eight columns of A, two 16-byte units (256 bytes) of B
+#pragma unroll
+                    for (int j = 0; j < TM_WORDS; j++)
+                        if (j < words) {
+                            mma_i8_ts(d_tmem, at + j * 16, bd + j * wbox_units, idesc, c + j ? 1u : 0u);
+                            mma_i8_ts(d_tmem, at + j * 16 + 8, bd + j * wbox_units + 16, idesc, 1u);
+                        }
+                    umma_commit(&bar_empty[s]);
+                }
+                if (++s == TM_STAGES) { s = 0; par ^= 1u; }
+            }
+            if (ok && leader) umma_commit(&bar_acc_full[acc]);
+            __syncwarp();
+            if (++acc == naccs) { acc = 0; accpar ^= 1; first = 0; }
+        }
+    } else {
+        // =========================== epilogue ===========================
+        const int ew = warp - PW, group = ew >> 2, r0 = (warp & 3) * 32, ld = (int)ep.ld_out;
+        const float* const addsrc = ep.shortcut ? ep.shortcut : ep.accumulate ? ep.out : nullptr;
+        if (tid - PW * 32 < TC5_MAX_N) pop[tid - PW * 32] = (float)popw[tid - PW * 32] - EPI_POP_BIAS * TM_SCALE;
+        asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");
+        EpiWarp e;
+        e.init(epi_smem, ew);
+#pragma unroll
+        for (int k = 0; k < 4; k++) e.set_row(k, r0 + e.row_of(k), ld);
+        const EpiOut o{ep.out, nullptr, ep.bits, narrow};
+        const EpiChannels ch{pop, chan_a, chan_b};
+        // Items: 32-channel chunks of this CTA's tiles in order, dealt to the warp groups in turn.
+        const int nchunk = (n_this + 31) >> 5;
+        auto element = [&](int tile, int chunk) { return (size_t)tile * 128 * ld + n0 + chunk * 32 + e.q * 8; };
+        auto limit_of = [&](int tile, int chunk) { return chunk * 32 + e.q * 8 < n_this ? (uint32_t)(min(128, M - tile * 128) * ld) : 0u; };
+        int k = 0, chunk = group;
+        while (chunk >= nchunk) { chunk -= nchunk; k++; }
+        int tile = blockIdx.x + k * gridDim.x;
+        if (addsrc && tile < ntiles_m) {
+            const float* at = addsrc + element(tile, chunk);
+            const uint32_t limit = limit_of(tile, chunk);
+#pragma unroll
+            for (int s = 0; s < 4; s++) e.fetch(s, at, limit, narrow);
+        }
+        while (tile < ntiles_m) {
+            int k2 = k, chunk2 = chunk + EGROUPS;   // the item after this one, for the shortcut's prefetch
+            while (chunk2 >= nchunk) { chunk2 -= nchunk; k2++; }
+            const int tile2 = blockIdx.x + k2 * gridDim.x;
+            const int acc = k & (naccs - 1), cl = chunk * 32 + e.q * 8;
+            if (!mbar_wait_warp<64>(&bar_acc_full[acc], (k / naccs) & 1, abort_flag)) {
+                atomicCAS(&g_tc5_status, 0, 2);
+                s_abort = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            e.take(tmem_base + ((uint32_t)r0 << 16) + acc * acc_cols + chunk * 32);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_acc_empty[acc]);   // this warp's share of the accumulator has been read
+            if (addsrc)
+                e.finish<true, false, true>(o, ch, cl, element(tile, chunk), limit_of(tile, chunk), tile2 < ntiles_m ? addsrc + element(tile2, chunk2) : addsrc,
+                                            tile2 < ntiles_m ? limit_of(tile2, chunk2) : 0u);
+            else
+                e.finish<false, false, true>(o, ch, cl, element(tile, chunk), limit_of(tile, chunk), nullptr, 0u);
+            k = k2; chunk = chunk2; tile = tile2;
+        }
+    }
+
+    // ---- everybody is past its last use of the tensor memory ----
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == TM_WARPS) {
+        __syncwarp();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base));
+    }
+}
+
+}  // namespace dabnn

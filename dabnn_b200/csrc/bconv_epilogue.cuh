@@ -137,7 +137,7 @@ struct EpiWarp {
     // pixel at the lane's first channel, limit: elements from there on that exist (0 where the channels do not).  next /
     // next_limit: what `fetch` needs for the item to come.  KEEP: the results also stay in the buffer, at the places the
     // accumulators had.
-    template <bool SC, bool KEEP>
+    template <bool SC, bool KEEP, bool SCALED = false>
     __device__ __forceinline__ void finish(const EpiOut& o, const EpiChannels& ch, int cl, size_t e0, uint32_t limit, const float* next, uint32_t next_limit) {
         __syncwarp();
         float pop[8], a[8], b[8];
@@ -161,8 +161,9 @@ struct EpiWarp {
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 // an integer of less than 22 bits added to the bits of 1.5 * 2^23 is 1.5 * 2^23 + that integer as a float, and
-                // the sum with popcount - 1.5 * 2^23 is exact
-                y[i] = __fadd_rn(__uint_as_float(t[i] + 0x4B400000u), pop[i]);
+                // the sum with popcount - 1.5 * 2^23 is exact (SCALED: accumulators of 128 a bit, the bias in pop scaled alike)
+                const float f = __uint_as_float(t[i] + 0x4B400000u);
+                y[i] = SCALED ? __fmaf_rn(f, 1.f / 128.f, pop[i]) : __fadd_rn(f, pop[i]);
                 y[i] = __fadd_rn(__fmul_rn(a[i], y[i]), b[i]);
                 if (SC) y[i] = __fadd_rn(sc[s][i], y[i]);
             }

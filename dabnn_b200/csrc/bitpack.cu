@@ -8,6 +8,7 @@ namespace dabnn {
 // 32-bit half word, so a warp turns 512 contiguous input bytes into 16 output bytes per step.
 __global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ in, uint32_t* __restrict__ out,
                                                    size_t n4) {
+    grid_launch_dependents();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
     // n4 is a multiple of 16 (64 floats per word), so whole 8-lane groups are in or out together;
@@ -87,6 +88,7 @@ __global__ void im2col_kernel(const uint32_t* __restrict__ in, uint32_t* __restr
 __global__ void __launch_bounds__(256) fused_binarize_im2col_kernel(
     const float* __restrict__ in, uint32_t* __restrict__ col, int n, int h, int w, int c, int kh, int kw,
     int pad_h, int pad_w, int stride_h, int stride_w, int dil_h, int dil_w, int oh, int ow, int row_u32) {
+    grid_launch_dependents();
     const int lane = threadIdx.x & 31;
     const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -116,6 +118,7 @@ __global__ void __launch_bounds__(256) fused_binarize_im2col_kernel(
 __global__ void __launch_bounds__(256) fused_binarize_im2col_vec4_kernel(
     const float* __restrict__ in, uint32_t* __restrict__ col, int n, int h, int w, int c, int kh, int kw,
     int pad_h, int pad_w, int stride_h, int stride_w, int dil_h, int dil_w, int oh, int ow, int row_u32) {
+    grid_launch_dependents();
     const uint32_t per_row = (uint32_t)row_u32 * 8u;              // nibbles per output row
     const uint32_t total = (uint32_t)n * oh * ow * per_row;       // a multiple of 32
     const int len = kh * kw * c;

@@ -1,8 +1,9 @@
 // C-ABI entry points built on the binary contraction core: bgemm, bconv, the fused residual
 // block and the BinConv operator.
 #include <algorithm>
+#include <cmath>
 
-#include "bcontract_tc5.cuh"
+#include "bcontract_tmem.cuh"
 #include "kernels.h"
 
 namespace dabnn {
@@ -46,15 +47,15 @@ static int launch_engine(const XOp& xop, const WOp& wop, const EpilogueParams& e
 }
 
 // tcgen05 engine: persistent warp-specialised CTAs, one per SM (it owns all of the SM's tensor memory)
-template <int CW, class XOp, class WOp>
-static int launch_tc5_cw(const XOp& xop, const WOp& wop, const EpilogueParams& ep, int M, int N, int kwords,
+template <class XOp, class WOp>
+static int launch_tc5(const XOp& xop, const WOp& wop, const EpilogueParams& ep, int M, int N, int kwords,
                          cudaStream_t stream) {
-    auto kern = bcontract_tc5_kernel<CW, XOp, WOp>;
+    auto kern = bcontract_tc5_kernel<XOp, WOp>;
     static thread_local int configured_device = -1;
     int dev = 0;
     DABNN_CUDA_OK(cudaGetDevice(&dev));
     if (configured_device != dev) {
-        DABNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Tc5Cfg<CW>::TOTAL));
+        DABNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Tc5Cfg::TOTAL));
         configured_device = dev;
     }
     const int tiles_m = (M + 127) / 128, tiles_n = (N + TC5_MAX_N - 1) / TC5_MAX_N;
@@ -67,14 +68,67 @@ static int launch_tc5_cw(const XOp& xop, const WOp& wop, const EpilogueParams& e
         g_last_engine = DABNN_ENGINE_IMMA;
         return launch_engine<ENG_IMMA>(xop, wop, ep, M, N, kwords, stream);   // no TMA descriptor: the mma.sync engine
     }
-    kern<<<grid, TC5_THREADS, Tc5Cfg<CW>::TOTAL, stream>>>(xop, wop, ep, M, N, kwords, tiles_m, out_map);
+    kern<<<grid, TC5_THREADS, Tc5Cfg::TOTAL, stream>>>(xop, wop, ep, M, N, kwords, tiles_m, out_map);
     return check_launch("bcontract_tc5_kernel");
 }
-template <class XOp, class WOp>
-static int launch_tc5(const XOp& xop, const WOp& wop, const EpilogueParams& ep, int M, int N, int kwords,
-                      cudaStream_t stream) {
-    return tc5_chunk_words(kwords) == 2 ? launch_tc5_cw<2>(xop, wop, ep, M, N, kwords, stream)
-                                        : launch_tc5_cw<4>(xop, wop, ep, M, N, kwords, stream);
+// ---- TCGEN05 engine with the pixel operand in tensor memory ----
+constexpr int TMEM_SMEM_LIMIT = 229000;   // 227 KB less the kernel's static shared memory
+
+// Chooses between this kernel (and its channel block) and the one of bcontract_tc5.cuh by the time each should take, in ns: rounds
+// of the CTAs over the pixel tiles x the slower of K and epilogue per tile.  The constants are fits to a B200 at 24 shapes with
+// each setting forced (block x words of K):
+//   * a word of K costs 76 - 80 ns at 16 and 32 channels (the producers), 95 - 100 at 64, about 130 at 128 (the MMAs);
+//   * the epilogue costs 0.7 us a tile at 16 channels, 1.0 at 32, 1.6 at 64, 2.9 at 128;
+//   * the other kernel needs 268 ns a word at its 128 channels.
+// The channel block is halved until the filters fit into shared memory; from 41 words of K on only 32 channels do, every tile is
+// expanded N / 32 times, and a large M is better off without: 12544 x 512 x 4608 takes 63 us here and 58 there, 49 x 512 x 4608
+// 10.5 and 25.  At up to 40 words it is 40 us here and 59 there (50176 x 256 x 2304).
+// Producer warps: 4 for up to eight words of K, where the epilogue is what takes the time (50176 x 512 x 256: 27.4 us, 30.6 with
+// 8), else 8 (200704 x 128 x 1152: 53.6 us, 55.8 with 4, 802816 x 64 x 576 as a convolution 98 and 135); 12 only where the
+// epilogue's buffers would not leave room for 16 channels of filters.  Up to 20 words 128 channels fit, and this kernel was the
+// faster one wherever that was measured.
+static bool tmem_plan(const EpilogueParams& ep, int M, int N, int kwords, TmemPlan* best) {
+    if (kwords > TM_MAX_WORDS || ep.ld_out >= TM_MAX_LD || (ep.shortcut && ep.ld_sc != ep.ld_out) ||
+        (ep.bits && (ep.ld_out != N || ep.ld_bits * 64 != N)))
+        return false;
+    const double tiles_m = (M + 127) / 128;
+    auto rounds = [&](int channels) { return std::ceil(tiles_m / std::max(1, sm_count() / ((N + channels - 1) / channels))); };
+    double best_ns = rounds(TC5_MAX_N) * kwords * 268.;
+    best->nbc = 0;
+    for (int nbc = 128; nbc >= (ep.bits ? 32 : 16); nbc >>= 1) {
+        if (nbc > 16 && nbc / 2 >= N) continue;
+        int pw = kwords <= 8 ? 4 : 8;
+        if (nbc == 16 && tmem_smem_bytes(nbc, kwords, pw) > TMEM_SMEM_LIMIT) pw = 12;
+        if (tmem_smem_bytes(nbc, kwords, pw) > TMEM_SMEM_LIMIT) continue;
+        const double word_ns = nbc == 128 ? 130. : nbc == 64 ? 95. : 78., filters_ns = 0.15 * kwords * nbc;
+        const double ns = rounds(nbc) * std::max(kwords * word_ns, 350. + 20. * nbc) + filters_ns;
+        if (ns < best_ns || (!best->nbc && kwords <= 20)) { *best = TmemPlan{nbc, pw}; best_ns = ns; }
+    }
+    return best->nbc != 0;
+}
+
+template <int PW, class XOp, class WOp>
+static int launch_tmem(const TmemPlan& plan, const XOp& xop, const WOp& wop, const EpilogueParams& ep, int M, int N, int kwords,
+                       cudaStream_t stream, bool after_pack) {
+    auto kern = bcontract_tmem_kernel<PW, XOp, WOp>;
+    static thread_local int configured_device = -1;
+    int dev = 0;
+    DABNN_CUDA_OK(cudaGetDevice(&dev));
+    if (configured_device != dev) {
+        DABNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TMEM_SMEM_LIMIT));
+        configured_device = dev;
+    }
+    const int tiles_m = (M + 127) / 128, tiles_n = (N + plan.nbc - 1) / plan.nbc, per_n = std::max(1, sm_count() / tiles_n);
+    const dim3 grid(std::min(tiles_m, per_n), tiles_n);
+    auto al32 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; };
+    const int narrow = !(ep.ld_out % 8 == 0 && al32(ep.out) && al32(ep.shortcut));
+    const size_t smem = tmem_smem_bytes(plan.nbc, kwords, PW);
+    if (after_pack) {
+        DABNN_CUDA_OK(launch_overlapped(kern, grid, dim3(TM_THREADS), smem, stream, xop, wop, ep, M, N, kwords, tiles_m, plan.nbc, narrow, 1));
+    } else {
+        kern<<<grid, TM_THREADS, smem, stream>>>(xop, wop, ep, M, N, kwords, tiles_m, plan.nbc, narrow, 0);
+    }
+    return check_launch("bcontract_tmem_kernel");
 }
 
 static bool tc5_eligible(const EpilogueParams& ep, int N) {
@@ -85,14 +139,22 @@ static bool tc5_eligible(const EpilogueParams& ep, int N) {
 
 template <class XOp, class WOp>
 int launch_bcontract(int engine, const XOp& xop, const WOp& wop, const EpilogueParams& ep, int M, int N,
-                     int kwords, cudaStream_t stream) {
+                     int kwords, cudaStream_t stream, bool after_pack = false) {
     if (M <= 0 || N <= 0) return DABNN_OK;
     DABNN_REQUIRE(kwords < (1 << 17), DABNN_ERR_SHAPE, "contraction: K must be below 2^23 bits");
     if (engine == DABNN_ENGINE_AUTO) engine = DABNN_ENGINE_TCGEN05;
     if (engine == DABNN_ENGINE_TCGEN05 && !tc5_eligible(ep, N)) engine = DABNN_ENGINE_IMMA;
     g_last_engine = engine;
     switch (engine) {
-        case DABNN_ENGINE_TCGEN05: return launch_tc5(xop, wop, ep, M, N, kwords, stream);
+        case DABNN_ENGINE_TCGEN05: {
+            TmemPlan plan;
+            if (!tmem_plan(ep, M, N, kwords, &plan)) return launch_tc5(xop, wop, ep, M, N, kwords, stream);
+            switch (plan.producer_warps) {
+                case 4: return launch_tmem<4>(plan, xop, wop, ep, M, N, kwords, stream, after_pack);
+                case 8: return launch_tmem<8>(plan, xop, wop, ep, M, N, kwords, stream, after_pack);
+                default: return launch_tmem<12>(plan, xop, wop, ep, M, N, kwords, stream, after_pack);
+            }
+        }
         case DABNN_ENGINE_POPC: return launch_engine<ENG_POPC>(xop, wop, ep, M, N, kwords, stream);
         case DABNN_ENGINE_B1: return launch_engine<ENG_B1>(xop, wop, ep, M, N, kwords, stream);
         case DABNN_ENGINE_IMMA: return launch_engine<ENG_IMMA>(xop, wop, ep, M, N, kwords, stream);
@@ -138,17 +200,15 @@ int bconv_expand_weights(const uint64_t* weight, size_t weight_words, int cout, 
                   "expand_weights: filter rows shorter than kwords");
     DABNN_REQUIRE((reinterpret_cast<uintptr_t>(dst) & 15) == 0, DABNN_ERR_ARG, "expand_weights: dst must be 16-byte aligned");
     RowMajorOperand wop{weight, (long long)(weight_words / cout), cout, kwords};
-    const int cw = tc5_chunk_words(kwords);
-    dim3 grid((kwords + cw - 1) / cw, (cout + TC5_MAX_N - 1) / TC5_MAX_N);
-    if (cw == 2) tc5_expand_weights_kernel<2><<<grid, 256, 0, stream>>>(wop, cout, kwords, dst);
-    else tc5_expand_weights_kernel<4><<<grid, 256, 0, stream>>>(wop, cout, kwords, dst);
+    dim3 grid((kwords + Tc5Cfg::WORDS - 1) / Tc5Cfg::WORDS, (cout + TC5_MAX_N - 1) / TC5_MAX_N);
+    tc5_expand_weights_kernel<<<grid, 256, 0, stream>>>(wop, cout, kwords, dst);
     return check_launch("tc5_expand_weights_kernel");
 }
 
 int bconv_block_impl(const uint64_t* in_bits, const uint64_t* weight, size_t weight_words, const float* a,
                      const float* b, const float* shortcut, float* out_f32, uint64_t* out_bits, int n, int h,
                      int w, int cw, int cout, int kh, int kw, int pad_h, int pad_w, int stride_h,
-                     int stride_w, int engine, cudaStream_t stream, const unsigned char* w_expanded) {
+                     int stride_w, int engine, cudaStream_t stream, const unsigned char* w_expanded, bool after_pack) {
     int rc = check_conv_args(in_bits, weight, weight_words, n, h, w, cw, cout, kh, kw, pad_h, pad_w, stride_h,
                              stride_w);
     if (rc) return rc;
@@ -158,7 +218,7 @@ int bconv_block_impl(const uint64_t* in_bits, const uint64_t* weight, size_t wei
     const ConvOperand xop = make_conv_operand(in_bits, n, h, w, cw, kh, kw, pad_h, pad_w, stride_h, stride_w);
     RowMajorOperand wop{weight, (long long)(weight_words / cout), cout, xop.kwords};
     EpilogueParams ep{out_f32, cout, 0, a, b, shortcut, cout, out_bits, cout / 64, w_expanded};
-    return launch_bcontract(engine, xop, wop, ep, xop.rows, cout, xop.kwords, stream);
+    return launch_bcontract(engine, xop, wop, ep, xop.rows, cout, xop.kwords, stream, after_pack);
 }
 
 }  // namespace dabnn
@@ -229,8 +289,8 @@ extern "C" int dabnn_binconv_forward(const float* in, const uint64_t* weight, si
         // rows (OnnxConverter.cpp:121-156); both are "at least kh*kw*cw words per filter" here
         int rc = dabnn_pack_mat(in, ws, n, h, w, cin, s);
         if (rc) return rc;
-        return dabnn_bconv(ws, weight, weight_words, out, n, h, w, cin / 64, cout, kh, kw, pad_h, pad_w,
-                           stride_h, stride_w, engine, s);
+        return bconv_block_impl(ws, weight, weight_words, nullptr, nullptr, nullptr, out, nullptr, n, h, w, cin / 64, cout, kh, kw,
+                                pad_h, pad_w, stride_h, stride_w, engine, static_cast<cudaStream_t>(s), nullptr, true);
     }
     const int oh = conv_out_dim(h, pad_h, 1, kh, stride_h), ow = conv_out_dim(w, pad_w, 1, kw, stride_w);
     const int row_words = (int)(((size_t)kh * kw * cin + 127) / 128 * 2);
@@ -241,7 +301,7 @@ extern "C" int dabnn_binconv_forward(const float* in, const uint64_t* weight, si
     RowMajorOperand xop{ws, row_words, n * oh * ow, row_words};
     RowMajorOperand wop{weight, row_words, cout, row_words};
     EpilogueParams ep{out, cout, 0, nullptr, nullptr, nullptr, 0, nullptr, 0};
-    return launch_bcontract(engine, xop, wop, ep, n * oh * ow, cout, row_words, static_cast<cudaStream_t>(s));
+    return launch_bcontract(engine, xop, wop, ep, n * oh * ow, cout, row_words, static_cast<cudaStream_t>(s), true);
 }
 
 int dabnn::contraction_status_word(int** addr) {

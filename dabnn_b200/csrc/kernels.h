@@ -32,11 +32,13 @@ bool make_u8_tensor_map(CUtensorMap_st* map, const unsigned char* base, int rank
 size_t bconv_expanded_weight_bytes(int cout, int kwords);
 int bconv_expand_weights(const uint64_t* weight, size_t weight_words, int cout, int kwords, unsigned char* dst,
                          cudaStream_t stream);
-// bconv + optional affine + optional shortcut + optional sign-bit output (see dabnn_bconv_block).
+// bconv + optional affine + optional shortcut + optional sign-bit output (see dabnn_bconv_block).  after_pack: the launch
+// before it in the stream is one of bitpack.cu's kernels, itself launched without overlap, that wrote in_bits and nothing
+// else this call reads.
 int bconv_block_impl(const uint64_t* in_bits, const uint64_t* weight, size_t weight_words, const float* a,
                      const float* b, const float* shortcut, float* out_f32, uint64_t* out_bits, int n, int h,
                      int w, int cw, int cout, int kh, int kw, int pad_h, int pad_w, int stride_h,
-                     int stride_w, int engine, cudaStream_t stream, const unsigned char* w_expanded = nullptr);
+                     int stride_w, int engine, cudaStream_t stream, const unsigned char* w_expanded = nullptr, bool after_pack = false);
 
 // Byte-activation engine (bconv_u8.cuh): activations as {0,1} bytes in NHWC, fed to the tensor cores by TMA.
 // bconv_u8_supported: whether the shape is taken (and its tensor maps can be encoded on this driver).

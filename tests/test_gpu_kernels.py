@@ -276,6 +276,37 @@ def test_bconv_block_fused_equals_layer_sequence(ops, port, engine, H, cin, cout
     assert torch.equal(b2, b3)
 
 
+# n, h, w, words of channels, cout, k, pad, stride: every channel block (128 ... 16 and the kernel for longer K), stages and pixel tiles
+# that end early, odd and even words per tap, channels that end inside a 32-channel item
+@pytest.mark.parametrize("n,h,w,cw,cout,k,pad,stride", [
+    (1, 1, 1, 1, 16, 1, 0, 1), (1, 127, 1, 4, 128, 1, 0, 1), (1, 43, 3, 5, 144, 1, 0, 1), (150, 16, 8, 8, 64, 1, 0, 1),
+    (150, 16, 8, 1, 128, 1, 0, 1), (601, 8, 8, 2, 128, 3, 1, 1), (3, 11, 13, 3, 48, 3, 1, 2), (2, 14, 14, 4, 192, 3, 1, 1),
+    (1, 7, 7, 8, 512, 3, 1, 1), (150, 8, 8, 4, 256, 3, 1, 1), (1, 9, 9, 5, 80, 5, 2, 1), (2, 9, 7, 8, 32, 5, 2, 2),
+    (1, 5, 5, 9, 16, 5, 2, 1), (64, 14, 14, 8, 512, 3, 1, 1)])
+def test_bconv_tensor_memory_kernels(ops, port, n, h, w, cw, cout, k, pad, stride):
+    rng = np.random.default_rng(h * 100 + cout)
+    x, wt = rand_bits(rng, (n, h, w, cw)), rand_bits(rng, cout * k * k * cw)
+    oh, ow = (h + 2 * pad - k) // stride + 1, (w + 2 * pad - k) // stride + 1
+    a, b = rng.uniform(-0.1, 0.1, cout).astype(np.float32), rng.normal(0, 1, cout).astype(np.float32)
+    sc = rng.normal(0, 1, (n, oh, ow, cout)).astype(np.float32)
+    xd, wd = dev_bits(x), dev_bits(wt)
+    layer = (xd, wd, cout, k, k, pad, pad, stride, stride)
+    cnt = ops.bconv(*layer, "tcgen05")
+    assert ops.last_engine() == "tcgen05" and torch.equal(cnt, ops.bconv(*layer, "popc"))
+    # a shortcut that starts on a 16-byte boundary only
+    buf = torch.empty(sc.size + 4, device="cuda")
+    buf[4:] = dev_f32(sc).flatten()
+    for shortcut in (dev_f32(sc), buf[4:].view(sc.shape)):
+        f32, bits = ops.bconv_block(*layer, dev_f32(a), dev_f32(b), shortcut, want_f32=True, want_bits=cout % 64 == 0, engine="tcgen05")
+        for i in sorted({0, n // 2, n - 1}):
+            exp_cnt = port.baseline_bconv(x[i], wt, cout, k, k, pad, pad, stride, stride)
+            exp = port.add(port.affine(exp_cnt, a, b), sc[i])
+            assert same_bits(host(cnt[i]), exp_cnt) and same_bits(host(f32[i]), exp)
+            if cout % 64 == 0:
+                assert same_bits(host_bits(bits[i]), port.pack_mat(exp))
+    assert ops.engine_status() == 0
+
+
 # ------------------------------------------------------------------------------------ byte-activation engine
 U8_SHAPES = [  # n, H, W, cin, cout, k, pad, stride
     (3, 14, 14, 64, 64, 3, 1, 1),      # whole images per tile would not fit: two tiles of 7 rows
