@@ -41,6 +41,17 @@ def test_pack_random(ops, port, shape):
     assert same_bits(host_bits(ops.pack_mat(dev_f32(x))), port.pack_mat(x))
 
 
+@pytest.mark.parametrize("offset", [0, 4, 8])   # 32-byte and 16-byte boundaries: two kernels
+@pytest.mark.parametrize("size", [64, 960, 1024, 1088, 4096 + 64, 3 * 148 * 8 * 1024 * 8 + 192])
+def test_pack_alignments_and_tails(ops, port, size, offset):
+    rng = np.random.default_rng(size + offset)
+    x = rng.normal(0, 1, size).astype(np.float32)
+    x[rng.random(size) < 0.02] = rng.choice(np.array([0.0, -0.0, np.nan, np.inf, -np.inf, 1e-45], np.float32), 1)
+    buf = torch.zeros(size + 16, device="cuda")
+    buf[offset:offset + size] = dev_f32(x)
+    assert same_bits(host_bits(ops.pack_mat(buf[offset:offset + size].view(1, 1, 1, size))).ravel(), port.pack_64(x).ravel())
+
+
 def test_pack_large_matches_torch_property(ops):
     """Full-size check at the batch-256 operand of the bgemm config: popcount of the packed words
     equals the number of positive inputs, and unpacking word 0 reproduces the signs."""
