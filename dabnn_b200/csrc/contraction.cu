@@ -74,37 +74,39 @@ static int launch_tc5(const XOp& xop, const WOp& wop, const EpilogueParams& ep, 
 // ---- TCGEN05 engine with the pixel operand in tensor memory ----
 constexpr int TMEM_SMEM_LIMIT = 229000;   // 227 KB less the kernel's static shared memory
 
-// Chooses between this kernel (and its channel block) and the one of bcontract_tc5.cuh by the time each should take, in ns: rounds
-// of the CTAs over the pixel tiles x the slower of K and epilogue per tile.  The constants are fits to a B200 at 24 shapes with
-// each setting forced (block x words of K):
-//   * a word of K costs 76 - 80 ns at 16 and 32 channels (the producers), 95 - 100 at 64, about 130 at 128 (the MMAs);
-//   * the epilogue costs 0.7 us a tile at 16 channels, 1.0 at 32, 1.6 at 64, 2.9 at 128;
-//   * the other kernel needs 268 ns a word at its 128 channels.
-// The channel block is halved until the filters fit into shared memory; from 41 words of K on only 32 channels do, every tile is
-// expanded N / 32 times, and a large M is better off without: 12544 x 512 x 4608 takes 63 us here and 58 there, 49 x 512 x 4608
-// 10.5 and 25.  At up to 40 words it is 40 us here and 59 there (50176 x 256 x 2304).
+// What the epilogue and the accumulators of these kernels take; the rest is left to the kernel of bcontract_tc5.cuh.
+static bool tmem_takes(const EpilogueParams& ep, int N, int kwords) {
+    return kwords <= TM_MAX_WORDS && ep.ld_out < TM_MAX_LD && (!ep.shortcut || ep.ld_sc == ep.ld_out) &&
+           (!ep.bits || (ep.ld_out == N && ep.ld_bits * 64 == N));
+}
+
+// Chooses between resident filters (and their channel block) and streamed ones (nbc = 0) by the time each should take, in ns:
+// rounds of the CTAs over the pixel tiles x the slower of K and epilogue per tile.  The constants are fits to a B200 at 36 shapes
+// with each setting forced:
+//   * a word of K costs 76 - 110 ns a tile at 16 and 32 channels (the producers; GEMM rows and convolutions), 95 - 125 at 64,
+//     about 130 at 128 (the MMAs), and 107 - 140 with streamed filters, whose ring takes 6 us more to fill;
+//   * the epilogue costs 0.7 us a tile at 16 channels, 1.0 at 32, 1.6 at 64, 2.9 at 128.
+// Up to 20 words of K 128 channels fit, and resident filters were always the faster ones.  From 41 words on only 32 channels fit:
+// streamed filters take 49.9 us for 12544 x 512 x 4608 where 32 resident channels take 63 and the kernel of bcontract_tc5.cuh 58,
+// and 353 us for 64 x 28x28x384 -> 512 5x5 (433); a few pixel tiles are better off with 16 resident channels on more SMs,
+// 49 x 512 x 4608: 10.5 us, 15.9 streamed.
 // Producer warps: 4 for up to eight words of K, where the epilogue is what takes the time (50176 x 512 x 256: 27.4 us, 30.6 with
 // 8), else 8 (200704 x 128 x 1152: 53.6 us, 55.8 with 4, 802816 x 64 x 576 as a convolution 98 and 135); 12 only where the
-// epilogue's buffers would not leave room for 16 channels of filters.  Up to 20 words 128 channels fit, and this kernel was the
-// faster one wherever that was measured.
-static bool tmem_plan(const EpilogueParams& ep, int M, int N, int kwords, TmemPlan* best) {
-    if (kwords > TM_MAX_WORDS || ep.ld_out >= TM_MAX_LD || (ep.shortcut && ep.ld_sc != ep.ld_out) ||
-        (ep.bits && (ep.ld_out != N || ep.ld_bits * 64 != N)))
-        return false;
+// epilogue's buffers would not leave room for 16 channels of filters.
+static TmemPlan tmem_plan(const EpilogueParams& ep, int M, int N, int kwords) {
     const double tiles_m = (M + 127) / 128;
     auto rounds = [&](int channels) { return std::ceil(tiles_m / std::max(1, sm_count() / ((N + channels - 1) / channels))); };
-    double best_ns = rounds(TC5_MAX_N) * kwords * 268.;
-    best->nbc = 0;
+    double best_ns = kwords <= 20 ? 1e30 : rounds(TS_NBC) * kwords * 120. + 6000.;
+    TmemPlan best{0, 0};
     for (int nbc = 128; nbc >= (ep.bits ? 32 : 16); nbc >>= 1) {
         if (nbc > 16 && nbc / 2 >= N) continue;
         int pw = kwords <= 8 ? 4 : 8;
         if (nbc == 16 && tmem_smem_bytes(nbc, kwords, pw) > TMEM_SMEM_LIMIT) pw = 12;
         if (tmem_smem_bytes(nbc, kwords, pw) > TMEM_SMEM_LIMIT) continue;
-        const double word_ns = nbc == 128 ? 130. : nbc == 64 ? 95. : 78., filters_ns = 0.15 * kwords * nbc;
-        const double ns = rounds(nbc) * std::max(kwords * word_ns, 350. + 20. * nbc) + filters_ns;
-        if (ns < best_ns || (!best->nbc && kwords <= 20)) { *best = TmemPlan{nbc, pw}; best_ns = ns; }
+        const double ns = rounds(nbc) * std::max(kwords * (nbc == 128 ? 130. : 95.), 350. + 20. * nbc) + 0.15 * kwords * nbc;
+        if (ns < best_ns) { best = TmemPlan{nbc, pw}; best_ns = ns; }
     }
-    return best->nbc != 0;
+    return best;
 }
 
 template <int PW, class XOp, class WOp>
@@ -131,6 +133,23 @@ static int launch_tmem(const TmemPlan& plan, const XOp& xop, const WOp& wop, con
     return check_launch("bcontract_tmem_kernel");
 }
 
+template <class XOp, class WOp>
+static int launch_tmem_stream(const XOp& xop, const WOp& wop, const EpilogueParams& ep, int M, int N, int kwords, cudaStream_t stream) {
+    auto kern = bcontract_tmem_stream_kernel<XOp, WOp>;
+    static thread_local int configured_device = -1;
+    int dev = 0;
+    DABNN_CUDA_OK(cudaGetDevice(&dev));
+    if (configured_device != dev) {
+        DABNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_BYTES));
+        configured_device = dev;
+    }
+    const int tiles_m = (M + 127) / 128, tiles_n = (N + TS_NBC - 1) / TS_NBC, per_n = std::max(1, sm_count() / tiles_n);
+    auto al32 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; };
+    const int narrow = !(ep.ld_out % 8 == 0 && al32(ep.out) && al32(ep.shortcut));
+    kern<<<dim3(std::min(tiles_m, per_n), tiles_n), TM_THREADS, TS_SMEM_BYTES, stream>>>(xop, wop, ep, M, N, kwords, tiles_m, narrow);
+    return check_launch("bcontract_tmem_stream_kernel");
+}
+
 static bool tc5_eligible(const EpilogueParams& ep, int N) {
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     return N % 16 == 0 && (!ep.out || (ep.ld_out % 4 == 0 && al16(ep.out))) &&
@@ -147,8 +166,9 @@ int launch_bcontract(int engine, const XOp& xop, const WOp& wop, const EpilogueP
     g_last_engine = engine;
     switch (engine) {
         case DABNN_ENGINE_TCGEN05: {
-            TmemPlan plan;
-            if (!tmem_plan(ep, M, N, kwords, &plan)) return launch_tc5(xop, wop, ep, M, N, kwords, stream);
+            if (!tmem_takes(ep, N, kwords)) return launch_tc5(xop, wop, ep, M, N, kwords, stream);
+            const TmemPlan plan = tmem_plan(ep, M, N, kwords);
+            if (!plan.nbc) return launch_tmem_stream(xop, wop, ep, M, N, kwords, stream);
             switch (plan.producer_warps) {
                 case 4: return launch_tmem<4>(plan, xop, wop, ep, M, N, kwords, stream, after_pack);
                 case 8: return launch_tmem<8>(plan, xop, wop, ep, M, N, kwords, stream, after_pack);

@@ -29,6 +29,7 @@ bool make_u8_tensor_map(CUtensorMap_st* map, const unsigned char* base, int rank
 
 // Weights of a binary convolution expanded once to the TCGEN05 engine's stage layout (bytes {0,1}, 8x the packed
 // size): size of the buffer, and the kernel that fills it.  bconv_block_impl takes the buffer as w_expanded.
+// (Read by the kernel for K of more than 255 words; the others expand their filters as they go.)
 size_t bconv_expanded_weight_bytes(int cout, int kwords);
 int bconv_expand_weights(const uint64_t* weight, size_t weight_words, int cout, int kwords, unsigned char* dst,
                          cudaStream_t stream);

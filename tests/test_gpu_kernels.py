@@ -293,7 +293,8 @@ def test_bconv_block_fused_equals_layer_sequence(ops, port, engine, H, cin, cout
     (1, 1, 1, 1, 16, 1, 0, 1), (1, 127, 1, 4, 128, 1, 0, 1), (1, 43, 3, 5, 144, 1, 0, 1), (150, 16, 8, 8, 64, 1, 0, 1),
     (150, 16, 8, 1, 128, 1, 0, 1), (601, 8, 8, 2, 128, 3, 1, 1), (3, 11, 13, 3, 48, 3, 1, 2), (2, 14, 14, 4, 192, 3, 1, 1),
     (1, 7, 7, 8, 512, 3, 1, 1), (150, 8, 8, 4, 256, 3, 1, 1), (1, 9, 9, 5, 80, 5, 2, 1), (2, 9, 7, 8, 32, 5, 2, 2),
-    (1, 5, 5, 9, 16, 5, 2, 1), (64, 14, 14, 8, 512, 3, 1, 1)])
+    (1, 5, 5, 9, 16, 5, 2, 1), (64, 14, 14, 8, 512, 3, 1, 1),
+    (106, 14, 14, 8, 512, 3, 1, 1), (160, 12, 12, 3, 80, 5, 2, 1), (4, 6, 6, 12, 64, 5, 2, 1)])
 def test_bconv_tensor_memory_kernels(ops, port, n, h, w, cw, cout, k, pad, stride):
     rng = np.random.default_rng(h * 100 + cout)
     x, wt = rand_bits(rng, (n, h, w, cw)), rand_bits(rng, cout * k * k * cw)
