@@ -76,7 +76,7 @@ constexpr int TMEM_SMEM_LIMIT = 229000;   // 227 KB less the kernel's static sha
 
 // What the epilogue and the accumulators of these kernels take; the rest is left to the kernel of bcontract_tc5.cuh.
 static bool tmem_takes(const EpilogueParams& ep, int N, int kwords) {
-    return kwords <= TM_MAX_WORDS && ep.ld_out < TM_MAX_LD && (!ep.shortcut || ep.ld_sc == ep.ld_out) &&
+    return kwords >= 1 && kwords <= TM_MAX_WORDS && N <= 65535 * TS_NBC /* grid */ && ep.ld_out < TM_MAX_LD && (!ep.shortcut || ep.ld_sc == ep.ld_out) &&
            (!ep.bits || (ep.ld_out == N && ep.ld_bits * 64 == N));
 }
 
@@ -95,11 +95,14 @@ static bool tmem_takes(const EpilogueParams& ep, int N, int kwords) {
 // epilogue's buffers would not leave room for 16 channels of filters.
 static TmemPlan tmem_plan(const EpilogueParams& ep, int M, int N, int kwords) {
     const double tiles_m = (M + 127) / 128;
-    auto rounds = [&](int channels) { return std::ceil(tiles_m / std::max(1, sm_count() / ((N + channels - 1) / channels))); };
+    auto rounds = [&](int channels) {   // over the pixel tiles, times the waves that more channel blocks than SMs take
+        const int blocks = (N + channels - 1) / channels, sms = sm_count();
+        return std::ceil(tiles_m / std::max(1, sms / blocks)) * ((blocks + sms - 1) / sms);
+    };
     double best_ns = kwords <= 20 ? 1e30 : rounds(TS_NBC) * kwords * 120. + 6000.;
     TmemPlan best{0, 0};
     for (int nbc = 128; nbc >= (ep.bits ? 32 : 16); nbc >>= 1) {
-        if (nbc > 16 && nbc / 2 >= N) continue;
+        if ((nbc > 16 && nbc / 2 >= N) || N > 65535 * nbc) continue;
         int pw = kwords <= 8 ? 4 : 8;
         if (nbc == 16 && tmem_smem_bytes(nbc, kwords, pw) > TMEM_SMEM_LIMIT) pw = 12;
         if (tmem_smem_bytes(nbc, kwords, pw) > TMEM_SMEM_LIMIT) continue;
@@ -251,6 +254,7 @@ extern "C" int dabnn_bgemm(int m, int n, int k, const uint64_t* a, int lda, cons
     if (m == 0 || n == 0) return DABNN_OK;
     DABNN_REQUIRE(a && b && c, DABNN_ERR_ARG, "bgemm: null pointer");
     DABNN_REQUIRE(lda >= m && ldb >= k && ldc >= m, DABNN_ERR_SHAPE, "bgemm: leading dimension too small");
+    if (k == 0) return DABNN_OK;   // nothing to add (the kernels want at least one word of K)
     // pixels (reference n) are the row dimension of the contraction, channels (reference m) the columns
     RowMajorOperand xop{b, ldb, n, k};
     ColMajorOperand wop{a, lda, m, k};

@@ -126,6 +126,23 @@ def test_bgemm_vs_oracle(ops, port, engine, m, n, kk):
     assert same_bits(host(c), exp)
 
 
+def test_bgemm_without_words_of_k_adds_nothing(ops):
+    c0 = np.arange(48 * 5, dtype=np.float32)
+    word = dev_bits(np.full(64, 2**64 - 1, np.uint64))
+    for engine in ENGINES + ["auto"]:
+        c = dev_f32(c0)
+        ops.bgemm(48, 5, 0, word, 48, word, 1, c, 48, engine)
+        assert same_bits(host(c), c0), engine
+
+
+def test_bgemm_with_more_channel_blocks_than_sms(ops):
+    g = torch.Generator(device="cuda").manual_seed(5)
+    m, n, kk = 148 * 128 + 16, 300, 5
+    a, b = (torch.randint(-2**63, 2**63 - 1, (kk * x,), device="cuda", dtype=torch.int64, generator=g) for x in (m, n))
+    out = [ops.bgemm(m, n, kk, a, m, b, kk, torch.zeros(m * n, device="cuda"), m, e) for e in ("tcgen05", "popc")]
+    assert torch.equal(*out) and ops.engine_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(3136, 64, 576), (784, 128, 1152), (196, 256, 2304), (49, 512, 4608)])
 def test_bitpack_bgemm_config(ops, port, M, N, K):
     """Standalone bitpack + bgemm microbench shapes: fp32 operands sign-packed along K, then bgemm.
