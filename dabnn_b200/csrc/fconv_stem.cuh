@@ -39,12 +39,14 @@
 // With POOL the 3x3 stride-2 pad-1 max pooling that follows a ResNet stem happens in the same kernel and the stem's own
 // output never leaves the SM: a CTA's share is a run of POOLED rows, the stem rows under them arrive in order (the
 // first one computed again by the neighbour that shares it).  An epilogue thread meets the same pixel column in every
-// row, so it folds the window's rows in registers with the reference's `acc < t ? t : acc` rule; every second stem row
-// completes a pooled row, which alone is parked in the staging boxes, folded over its three columns and written out as
-// fp32 and as {0,1} sign bytes.  Affine and relu are applied to the completed maxima only (both are monotone per channel:
-// the sums are folded with their sign flipped where the affine's factor is negative).  The values are those of the two layers run one after the other (the maximum does not
-// depend on the order of the fold; the only freedom is which zero comes out of a window whose maximum is both +0 and
-// -0, where the reference's tap order is row-major and this one is column-major).
+// row, so it folds the window's rows in registers; every second stem row completes a pooled row, which alone is parked in
+// the staging boxes, folded over its three columns and written out as fp32 and as {0,1} sign bytes.  Affine and relu are
+// applied to the completed maxima only (both are monotone per channel: the sums are folded with their sign flipped where
+// the affine's factor is negative; fs_split covers the factors and shifts that could make a NaN of an infinite sum).  The
+// values are those of the layers run one after the other, whose fold `acc < t ? t : acc` starts at -FLT_MAX and never picks
+// a NaN: fmaxf drops NaNs as well, and a window without a number, or with nothing above -FLT_MAX, gives -FLT_MAX (the
+// maximum does not depend on the order of the fold; the only freedom is which zero comes out of a window whose maximum is
+// both +0 and -0).
 // Every wait is bounded; a wait that gives up records a code (31 converters, 32 / 33 MMA thread waiting for rows /
 // for an accumulator, 34 epilogue), raises the CTA's abort flag, and the CTA frees its tensor memory and returns.
 // Inputs must be finite: a non-finite pixel also poisons the output pixel whose zero-weight odd tap covers it.
@@ -83,19 +85,27 @@ __host__ __device__ inline int fs_smem_bytes(const FsGeom& g) {
 __device__ __forceinline__ void sts64(uint32_t addr, uint32_t x, uint32_t y) {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(x), "r"(y) : "memory");
 }
-// the reference's max-pool fold (MaxPool.cpp:209-246): keeps the earlier value on ties, never picks a NaN
-__device__ __forceinline__ float4 fs_sel(const float4 a, const float4 t) {
-    return make_float4(a.x < t.x ? t.x : a.x, a.y < t.y ? t.y : a.y, a.z < t.z ? t.z : a.z, a.w < t.w ? t.w : a.w);
+// POOL: a channel's affine a*y + b as two steps around the fold of the pooling, y -> before * y -> max -> after * max + b.
+// Ordinarily the factor's sign and its magnitude.  A factor that is zero or not finite comes first as a whole: its product
+// with an infinite (or zero) sum is a NaN, which the layers' pooling does not pick although the sum may be the largest one.
+// A shift of -inf makes a NaN of +inf only: the fold then runs the other way round and keeps the smallest product.
+__device__ __forceinline__ void fs_split(float a, float b, float& before, float& after) {
+    const bool whole = a == 0.f || !(fabsf(a) <= FLT_MAX);
+    before = whole ? a : copysignf(1.f, a);
+    after = whole ? 1.f : fabsf(a);
+    if (b < -FLT_MAX) { before = -before; after = -after; }
 }
-
-// affine (a: the factor's magnitude; its sign is in the value already) and relu of a pooled value
-__device__ __forceinline__ float4 fs_finish(float4 h, const float4 a, const float4 b, bool affine, int relu) {
+// the max-pool fold: drops NaNs
+__device__ __forceinline__ float4 fs_max(const float4 a, const float4 t) { return make_float4(fmaxf(a.x, t.x), fmaxf(a.y, t.y), fmaxf(a.z, t.z), fmaxf(a.w, t.w)); }
+// the second step, relu, and the start of the reference's fold (MaxPool.cpp:209-246), which only a larger value replaces
+__device__ __forceinline__ float4 fs_finish(float4 h, const float4 after, const float4 b, bool affine, int relu) {
     float v[4] = {h.x, h.y, h.z, h.w};
-    const float ka[4] = {a.x, a.y, a.z, a.w}, kb[4] = {b.x, b.y, b.z, b.w};
+    const float ka[4] = {after.x, after.y, after.z, after.w}, kb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         if (affine) v[e] = __fadd_rn(__fmul_rn(ka[e], v[e]), kb[e]);
         if (relu) v[e] = relu_ref(v[e]);
+        asm volatile("max.f32 %0, %0, 0fFF7FFFFF;" : "+f"(v[e]));   // -FLT_MAX as an immediate (in a register it makes the 7x7 form spill)
     }
     return make_float4(v[0], v[1], v[2], v[3]);
 }
@@ -143,7 +153,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_abort, epi_abort[2];
     __shared__ __align__(16) float chan_bias[FS_N], chan_a[FS_N], chan_b[FS_N];
-    __shared__ __align__(16) uint32_t chan_flip[FS_N];   // POOL: the sign bit where the affine's factor is negative
+    __shared__ __align__(16) float chan_first[FS_N];   // POOL: the affine's step before the fold; chan_a holds the one after it
 
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int n0 = blockIdx.y * FS_N;
@@ -193,8 +203,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
         chan_bias[tid] = (in && p.bias) ? __ldg(p.bias + n0 + tid) : 0.f;
         chan_a[tid] = (in && p.a) ? __ldg(p.a + n0 + tid) : 1.f;
         chan_b[tid] = (in && p.a) ? __ldg(p.b + n0 + tid) : 0.f;
-        chan_flip[tid] = __float_as_uint(chan_a[tid]) & 0x80000000u;
-        if (POOL) chan_a[tid] = fabsf(chan_a[tid]);
+        if (POOL) fs_split(chan_a[tid], chan_b[tid], chan_first[tid], chan_a[tid]);
     }
     // resident weights, K order (ky, kx < kxp, c < 4): element (n, k) -> (n / 8) * w_sbo + (k / 4) * 128 + (n % 8) * 16 + (k % 4) * 4
     // (four elements per thread and step, their loads issued together: the set-up is a fixed cost of every launch)
@@ -453,13 +462,13 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
 #pragma unroll
                         for (int q = 0; q < 2; q++) {
                             const int cl = cq * 16 + half * 8 + q * 4;
-                            const uint4 fl = *reinterpret_cast<const uint4*>(chan_flip + cl);
-                            const uint32_t f4[4] = {fl.x, fl.y, fl.z, fl.w};
+                            const float4 first = *reinterpret_cast<const float4*>(chan_first + cl);
+                            const float f4[4] = {first.x, first.y, first.z, first.w};
 #pragma unroll
                             for (int e = 0; e < 4; e++) {
                                 float f = __uint_as_float(y[q * 4 + e]) + __uint_as_float(xx[q * 4 + e]);   // + the hi*lo part
                                 if (p.bias) f = __fadd_rn(f, chan_bias[cl + e]);
-                                y[q * 4 + e] = __float_as_uint(f) ^ f4[e];
+                                y[q * 4 + e] = __float_as_uint(__fmul_rn(f, f4[e]));
                             }
                         }
                     }
@@ -517,13 +526,13 @@ __global__ void __launch_bounds__(FS_THREADS, 1)
                     const int k = (et & 255) + 256 * i;
                     const int px = k >> 3, q = k & 7;
                     if (k >= g.pw * 8 || h2 * 32 + q * 4 >= n_this) continue;
-                    float4 h = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
+                    float4 h = lds128f(sbox + 2 * px * 128 + ((q ^ (2 * px & 7)) << 4));
 #pragma unroll
-                    for (int dx = -1; dx <= 1; dx++) {   // the reference skips taps outside the image
+                    for (int dx = -1; dx <= 1; dx += 2) {   // the reference skips taps outside the image (the middle one is always inside)
                         const int ox = 2 * px + dx;
-                        if ((unsigned)ox < (unsigned)p.ow) h = fs_sel(h, lds128f(sbox + ox * 128 + ((q ^ (ox & 7)) << 4)));
+                        if ((unsigned)ox < (unsigned)p.ow) h = fs_max(h, lds128f(sbox + ox * 128 + ((q ^ (ox & 7)) << 4)));
                     }
-                    // (a product of the flipped sum and the factor's magnitude is the product of the two themselves)
+                    // (the product of the signed sum and the factor's magnitude is the product of the two themselves)
                     h = fs_finish(h, *reinterpret_cast<const float4*>(chan_a + h2 * 32 + q * 4), *reinterpret_cast<const float4*>(chan_b + h2 * 32 + q * 4),
                                   p.a != nullptr, p.relu);
                     const size_t e = (((size_t)img * g.ph + (oy >> 1)) * g.pw + px) * p.cout + n0 + h2 * 32 + q * 4;

@@ -692,6 +692,36 @@ def test_fconv_maxpool_fused_is_bit_identical(ops, port, n, h, cin, cout, ks, pa
         np.testing.assert_allclose(host(fused[i]), e, rtol=1e-4, atol=1e-4 * np.abs(e).max(), err_msg=f"image {i}")
 
 
+@pytest.mark.parametrize("factors", ["mixed", "none", "odd"])
+@pytest.mark.parametrize("relu", [True, False])
+@pytest.mark.parametrize("n,h,cin,cout,ks,pad", [(3, 224, 3, 64, 7, 3), (5, 130, 3, 48, 5, 2)])
+def test_fconv_maxpool_fused_signs_and_values_that_are_no_numbers(ops, n, h, cin, cout, ks, pad, relu, factors):
+    """The fused stem against its layers one after the other, bit for bit: factors of both signs, no affine, factors and
+    shifts that are zero or not finite; on ordinary images and on images with whole windows of NaN and infinities, whose
+    pooled value is the fold's start, -FLT_MAX (MaxPool.cpp:209-246)."""
+    rng = np.random.default_rng(h + cout + 2 * relu)
+    w = dev_f32(rng.normal(0, np.sqrt(2.0 / (cin * ks * ks)), (cout, ks, ks, cin)).astype(np.float32))
+    a = (rng.uniform(0.5, 1.5, cout) * rng.choice([-1, 1], cout)).astype(np.float32)
+    b, bias = rng.normal(0, 0.5, cout).astype(np.float32), rng.normal(0, 1, cout).astype(np.float32)
+    bias[7:10], bias[21] = (-np.inf, np.inf, np.nan), -np.inf    # with any pixels: sums of one infinity, or none that is a number
+    a[7], a[8] = 1.5, -0.5
+    if factors == "odd":
+        a[:6] = 0.0, -0.0, np.inf, -np.inf, np.nan, 1e-45
+        b[6], b[10], b[11], b[21], a[21] = np.inf, -np.inf, np.nan, np.inf, 0.0
+    affine = (None, None) if factors == "none" else (dev_f32(a), dev_f32(b))
+    x = rng.normal(0, 1, (n, h, h, cin)).astype(np.float32)
+    x[1, 20:70, 30:90] = np.nan
+    x[1, 100, 100] = np.inf
+    x[n - 1, 90:, :40], x[n - 1, 5, 7] = -np.inf, np.nan
+    fused, f8 = ops.fconv_maxpool(dev_f32(x), w, dev_f32(bias), pad, pad, 2, 2, *affine, relu, want_u8=True)
+    y = ops.fconv(dev_f32(x), w, dev_f32(bias), pad, pad, 2, 2)
+    y = y if factors == "none" else ops.affine_(y, *affine)
+    steps = ops.maxpool(ops.relu_(y) if relu else y, 3, 3, 1, 1, 2, 2)
+    assert ops.engine_status() == 0
+    assert torch.equal(fused, steps) and torch.equal(f8, (steps > 0).to(torch.uint8))
+    assert (steps == torch.finfo(torch.float32).min).any()
+
+
 def test_fconv_maxpool_refuses_other_shapes(ops):
     assert not ops.fconv_maxpool_supported(1, 64, 64, 3, 64, 7, 7, 3, 3, 2, 2)      # 32-pixel output rows: too short for the kernel
     assert not ops.fconv_maxpool_supported(1, 224, 224, 4, 64, 7, 7, 3, 3, 2, 2)    # more than three channels
