@@ -69,7 +69,9 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
     __shared__ __align__(8) uint64_t halo_full[HL_MAX_HSLOTS], halo_empty[HL_MAX_HSLOTS], w_full[HL_MAX_WSTAGES], w_empty[HL_MAX_WSTAGES];
     __shared__ __align__(8) uint64_t bar_acc_full[U8_ACCS], bar_acc_empty[U8_ACCS], bar_w;
     __shared__ uint32_t tmem_base_s;
-    __shared__ int s_abort, epi_abort;
+    // epi_abort: POOL, one flag per epilogue group.  Written by the group's own warps between its second barrier and its first,
+    // read between the first and the second: all four warps of a group read the same value and leave, or stay, together.
+    __shared__ int s_abort, epi_abort[EPI_GROUPS];
     __shared__ __align__(16) float pop[TC5_MAX_N];
     __shared__ __align__(16) float chan_a[TC5_MAX_N];
     __shared__ __align__(16) float chan_b[TC5_MAX_N];
@@ -101,7 +103,7 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
         mbar_init(&bar_w, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::);
         s_abort = 0;
-        epi_abort = 0;
+        for (int i = 0; i < EPI_GROUPS; i++) epi_abort[i] = 0;
     }
     if (p.imgs == 2 && tid < p.hslots * 4)   // the zero pixel behind the second image's halo (never written again)
         sts128(smem_u32(halo0) + (tid >> 2) * p.halo_stride + (p.img_pitch + (p.rows + 2) * p.P) * 64 + (tid & 3) * 16, 0u, 0u, 0u, 0u);
@@ -330,7 +332,7 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
                 if (!alive) {
                     atomicCAS(&g_u8_status, 0, 24);
                     s_abort = 1;
-                    epi_abort = 1;
+                    epi_abort[group] = 1;
                 } else {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     e.take(tmem_base + ((uint32_t)r0 << 16) + accbuf * acc_cols + chunk * 32);
@@ -347,7 +349,7 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
             if (POOL) {
                 // 2x2 average pooling of the item
                 group_sync();
-                if (epi_abort) break;
+                if (epi_abort[group]) break;
                 if (pchunk * 32 + pool_quad * 4 < n_this) {
                     const int img = per_img(ptile), oh0 = (ptile - img * p.tiles_per_img) * p.rows;
                     for (int pp = pool_px; pp < pool_pixels; pp += 16) {

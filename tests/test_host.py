@@ -155,3 +155,50 @@ def test_two_rank_gather_over_gloo(tmp_path):
                               stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True) for r in range(2)]
     outs = [p.communicate(timeout=180)[0] for p in procs]
     assert all(p.returncode == 0 for p in procs), outs
+
+
+def test_pooling_epilogue_never_strands_a_warp_at_a_barrier():
+    """The pooling epilogue of the halo kernel after a wait that gave up: groups of warps with barriers of their own, a flag
+    that makes a group leave.  Every interleaving of two groups of two warps over two items, with any subset of the waits
+    giving up, ends with all warps gone - none waits at a barrier that a warp of its group has left.  The order of the steps
+    and the flag's scope are read from the kernel."""
+    src = (ROOT / "dabnn_b200" / "csrc" / "bconv_halo.cuh").read_text()
+    steps, shared = [], False
+    for m in re.finditer(r"epi_abort(\[group\])? = 1;|if \(epi_abort(\[group\])?\) break;|group_sync\(\);", src):
+        steps.append("bar" if m[0].startswith("group_sync") else "read" if m[0].startswith("if") else "set")
+        shared |= steps[-1] != "bar" and "[group]" not in m[0]
+    assert steps == ["set", "bar", "read", "bar"]
+    program, groups, per = steps * 2, 2, 2
+    gone = len(program)
+
+    def successors(state):
+        pcs, arrived, flags = state
+        for w, pc in enumerate(pcs):
+            g = w // per
+            if pc == gone or w in arrived:
+                continue
+            move = lambda to: pcs[:w] + (to,) + pcs[w + 1:]
+            if program[pc] == "set":
+                yield move(pc + 1), arrived, flags
+                yield move(pc + 1), arrived, flags | {0 if shared else g}
+            elif program[pc] == "read":
+                yield move(gone if (0 if shared else g) in flags else pc + 1), arrived, flags
+            else:
+                there = arrived | {w}
+                mates = set(range(g * per, (g + 1) * per))
+                if mates <= there:   # the last one: the barrier opens
+                    yield tuple(p + 1 if v in mates else p for v, p in enumerate(pcs)), there - mates, flags
+                else:
+                    yield pcs, there, flags
+
+    start = ((0,) * (groups * per), frozenset(), frozenset())
+    seen, todo = {start}, [start]
+    while todo:
+        state = todo.pop()
+        following = list(successors(state))
+        assert following or all(pc == gone for pc in state[0]), f"stranded: {state}"
+        for s in following:
+            s = (s[0], frozenset(s[1]), frozenset(s[2]))
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
