@@ -37,12 +37,24 @@ constexpr int FG_THREADS = 32 + FG_CONVERTERS + 32 + FG_EPILOGUE;
 constexpr int FG_MMA_WARP = 1 + FG_CONVERTERS / 32;
 constexpr int FG_EPI_WARP0 = FG_MMA_WARP + 1;
 constexpr int FG_ACCS = 2;
-// The accumulators truncate, so every instruction that adds to them leaves a bias: 8e-9 of the result per k with three
-// instructions per slice in one accumulator (as on mma.sync), 5e-9 with the stacked form.  Up to this K the two stay
-// within 5e-6 of each other; beyond it the three-instruction form is kept, whose results are the mma.sync kernel's to 3e-6
-// (K = 12800) and which costs a fifth more operand reads.  Pointwise convolutions (short K, bound by HBM) keep it too: a
-// network binarises what follows them, and a sum that rounds the other way near zero flips a sign.
-constexpr int FG_STACKED_K = 2048;
+// The accumulators truncate: every instruction that adds to them leaves a bias, 8e-9 of the result per k with three
+// instructions per slice, 5e-9 with the stacked form.  So an accumulator takes one run of K only, and the epilogue adds the
+// runs in registers, rounded to nearest.  With runs of up to 36 stages the distance to the float64 result (2-norm, relative)
+// stays below 6e-6 at every K: 1.7e-6 at K = 288, 5.6e-6 at 1152, 5.4e-6 at 12800 (in one run of the three-instruction form:
+// 8.2e-5).  Each run more costs the tensor core about 450 cycles, while the epilogue reads the accumulators: 64 images of
+// 28x28x128 -> 128 3x3 take 71.9 us in one run, 73.2 in three, 75.0 in five; but the stacked form pays for them, 8 images of
+// 28x28x512 -> 128 5x5 376 us before, 338 in twelve runs.  A window whose taps end inside an 8-channel slice spends more
+// instructions than its K needs and gets two runs at least (3x3 of 20 channels: 1.36e-6 -> 0.90e-6, 27.7 -> 28.2 us; slices
+// that run across the taps, as in fconv_tc5.cuh: 1.24e-6).
+constexpr int FG_RUN = 36, FG_RUN_RAGGED = 18;   // stages per run at most
+inline int fg_runs(int taps, int cin) {
+    const int stages = taps * ((cin + FG_CHUNK - 1) / FG_CHUNK);
+    const bool ragged = taps * ((cin + 7) / 8) > (taps * cin + 7) / 8;
+    return ragged ? std::max(2, (stages + FG_RUN_RAGGED - 1) / FG_RUN_RAGGED) : (stages + FG_RUN - 1) / FG_RUN;
+}
+// The three-instruction form: pointwise convolutions of whole 32-channel groups up to K = 512 (bound by HBM).  A network
+// binarises what follows them, and a sum that rounds the other way near zero flips a sign.
+inline bool fg_stacked(bool pointwise, int cin) { return !pointwise || cin % FG_CHUNK || cin > 512; }
 constexpr int FG_TILE_BYTES = 128 * 128;       // 128 rows x 32 floats
 constexpr int FG_STAGE_BYTES = 4 * FG_TILE_BYTES;   // pixels hi, pixels lo, weights hi, weights lo
 constexpr int FG_MAX_STAGES = 3;
@@ -55,10 +67,31 @@ __device__ __forceinline__ uint64_t fg_desc_sw128(uint32_t saddr) {
 
 __host__ __device__ inline int fg_smem_bytes(int stages) { return 1024 + stages * FG_STAGE_BYTES + 2 * FG_TILE_BYTES; }
 
-template <bool STACKED>
+// COLS (8 or 16) accumulator columns of the warp's 32 rows, with the hi * W_lo half `lo` columns further added where there is one
+template <int COLS, bool STACKED>
+__device__ __forceinline__ void fg_take(float (&f)[COLS], uint32_t t_addr, uint32_t lo) {
+    uint32_t y[COLS], x[COLS];
+    auto ld = [](uint32_t (&v)[COLS], uint32_t at) {
+        if constexpr (COLS == 16)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                           "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(at));
+        else
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(at));
+    };
+    ld(y, t_addr);
+    if (STACKED) ld(x, t_addr + lo);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int e = 0; e < COLS; e++) f[e] = STACKED ? __fadd_rn(__uint_as_float(y[e]), __uint_as_float(x[e])) : __uint_as_float(y[e]);
+}
+
+// RUNS: K in more than one run (nruns; one otherwise)
+template <bool STACKED, bool RUNS>
 __global__ void __launch_bounds__(FG_THREADS, 1)
-    fconv_gemm_kernel(const FconvParams p, const int M, const int stages, const int n_blk, const int im2col, const __grid_constant__ CUtensorMap a_map,
-                      const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap wr_map, const __grid_constant__ CUtensorMap out_map) {
+    fconv_gemm_kernel(const FconvParams p, const int M, const int stages, const int n_blk, const int im2col, const int nruns,
+                      const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap wr_map, const __grid_constant__ CUtensorMap out_map) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t bar_loaded[FG_MAX_STAGES], bar_ready[FG_MAX_STAGES], bar_empty[FG_MAX_STAGES];
     __shared__ __align__(8) uint64_t bar_acc_full[FG_ACCS], bar_acc_empty[FG_ACCS];
@@ -74,6 +107,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
     const int tiles_m = (M + 127) / 128, nblocks = (p.cout + n_blk - 1) / n_blk;
     const uint32_t w_bytes = (uint32_t)n_blk * 128u;   // a weight tile of a stage
     const int nitems = tiles_m * nblocks;
+    const int run_len = nchunks / nruns, run_extra = nchunks - nruns * run_len;   // the first run_extra runs are a stage longer
     constexpr int ACC_COLS = 2 * FG_N;                  // hi * W_hi + lo * W_hi in the first n_blk columns, hi * W_lo in the next
     constexpr int TMEM_COLS = FG_ACCS * ACC_COLS;
 
@@ -184,19 +218,24 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
             const uint32_t idesc = idesc_m | ((uint32_t)(n_blk >> 3) << 17), idesc2 = idesc_m | ((uint32_t)(n_blk >> 2) << 17);
             uint32_t s = 0, par = 0;
             bool ok = true;
-            int i = 0;
-            for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, i++) {
-                const int accbuf = i % FG_ACCS, accuse = i / FG_ACCS;
-                if (accuse >= 1 && !mbar_wait_warp(&bar_acc_empty[accbuf], (accuse - 1) & 1, abort_flag)) {
-                    atomicCAS(&g_tc5_status, 0, 43);
-                    s_abort = 1;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d_tmem = tmem_base + accbuf * ACC_COLS;
-                uint32_t accum = 0;
-                int cg = 0;
+            int i = 0;   // runs so far: run i accumulates in accumulator i % FG_ACCS
+            for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+                uint32_t accum = 0, d_tmem = 0;
+                int cg = 0, run = 0, left_in_run = 0;
                 for (int c = 0; c < nchunks; c++) {
+                    if (left_in_run == 0) {
+                        const int accbuf = i % FG_ACCS, accuse = i / FG_ACCS;
+                        if (accuse >= 1 && !mbar_wait_warp(&bar_acc_empty[accbuf], (accuse - 1) & 1, abort_flag)) {
+                            atomicCAS(&g_tc5_status, 0, 43);
+                            s_abort = 1;
+                            ok = false;
+                            break;
+                        }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        d_tmem = tmem_base + accbuf * ACC_COLS;
+                        accum = 0;
+                        left_in_run = run_len + (run++ < run_extra ? 1 : 0);
+                    }
                     if (!mbar_wait_warp(&bar_ready[s], par, abort_flag)) {
                         atomicCAS(&g_tc5_status, 0, 44);
                         s_abort = 1;
@@ -217,19 +256,20 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                     };
                     const int left = p.cin - cg * FG_CHUNK;
                     if (leader) {
-                    if (left >= FG_CHUNK) {
+                        if (left >= FG_CHUNK) {
 #pragma unroll
-                        for (int j = 0; j < FG_CHUNK / 8; j++) slice(j);
-                    } else {   // the last channel group of a tap: only the slices that hold channels
-                        for (int j = 0; j * 8 < left; j++) slice(j);
+                            for (int j = 0; j < FG_CHUNK / 8; j++) slice(j);
+                        } else {   // the last channel group of a tap: only the slices that hold channels
+                            for (int j = 0; j * 8 < left; j++) slice(j);
+                        }
+                        umma_commit(&bar_empty[s]);
+                        if (left_in_run == 1) umma_commit(&bar_acc_full[i % FG_ACCS]);
                     }
-                    umma_commit(&bar_empty[s]);
-                    }
+                    if (--left_in_run == 0) i++;
                     if (++cg == cgroups) cg = 0;
                     accum = 1u;
                     if (++s == (uint32_t)stages) { s = 0; par ^= 1u; }
                 }
-                if (ok && leader) umma_commit(&bar_acc_full[accbuf]);
                 __syncwarp();
             }
         }
@@ -238,68 +278,58 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
         const int ew = warp - FG_EPI_WARP0, et = tid - FG_EPI_WARP0 * 32;
         const int r = (warp & 3) * 32 + lane, hq = ew >> 2;   // TMEM lane quarter of a warp = warp % 4; 16-channel quarter of the block
         const uint32_t stile_addr = smem_u32(stile);
+        const uint32_t t_mine = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + hq * 16;   // + accumulator + 64-channel block
         int i = 0;
-        bool alive = true;
-        for (int item = blockIdx.x; item < nitems && alive; item += gridDim.x, i++) {
-            const int tile = item / nblocks, nb = item - tile * nblocks;
-            const int n0 = nb * n_blk, n_this = min(n_blk, p.cout - n0);
-            const int accbuf = i % FG_ACCS, accuse = i / FG_ACCS;
-            const bool okw = __all_sync(0xffffffffu, mbar_wait<200>(&bar_acc_full[accbuf], accuse & 1, abort_flag));   // warp-uniform
+        bool alive = true, okw = true;
+        auto wait_run = [&]() {   // run i's accumulator
+            okw = mbar_wait_warp<200>(&bar_acc_full[i % FG_ACCS], (i / FG_ACCS) & 1, abort_flag);
             if (!okw) {
                 atomicCAS(&g_tc5_status, 0, 45);
                 s_abort = 1;
                 epi_abort = 1;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        };
+        auto release_run = [&]() {   // it is in registers: the MMA warp may reuse it
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_acc_empty[i % FG_ACCS]);
+        };
+        for (int item = blockIdx.x; item < nitems && alive; item += gridDim.x) {
+            const int tile = item / nblocks, nb = item - tile * nblocks;
+            const int n0 = nb * n_blk, n_this = min(n_blk, p.cout - n0);
             const int nblk64 = (n_this + 63) >> 6;
-            for (int blk = 0; blk < nblk64; blk++) {
+            // bias, affine, relu of 16 channels of 64-channel block blk, and its way out
+            auto write = [&](float (&v)[16], int blk) {
                 const int cb = blk * 64, width = min(64, n_this - cb);
                 const bool mine = width > hq * 16;
-                uint32_t v[16];
                 if (okw && mine) {
-                    const int c0 = cb + hq * 16;
-                    const uint32_t t_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + accbuf * ACC_COLS + c0;
-                    uint32_t x[16] = {};
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                                   "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                                 : "r"(t_addr));
-                    if (STACKED)
-                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]), "=r"(x[8]),
-                                   "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
-                                 : "r"(t_addr + n_blk));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int q = 0; q < 4; q++) {   // channel constants four at a time (Cout is a multiple of four)
-                        const int ch = min(n0 + c0 + q * 4, p.cout - 4);   // columns beyond Cout are clipped by the store
+                        const int ch = min(n0 + cb + hq * 16 + q * 4, p.cout - 4);   // columns beyond Cout are clipped by the store
                         float4 kb = make_float4(0.f, 0.f, 0.f, 0.f), ka = kb, kc = kb;
                         if (p.bias) kb = __ldg(reinterpret_cast<const float4*>(p.bias + ch));
                         if (p.a) { ka = __ldg(reinterpret_cast<const float4*>(p.a + ch)); kc = __ldg(reinterpret_cast<const float4*>(p.b + ch)); }
                         const float b4[4] = {kb.x, kb.y, kb.z, kb.w}, a4[4] = {ka.x, ka.y, ka.z, ka.w}, c4[4] = {kc.x, kc.y, kc.z, kc.w};
 #pragma unroll
                         for (int e = 0; e < 4; e++) {
-                            float f = __uint_as_float(v[q * 4 + e]);
-                            if (STACKED) f = __fadd_rn(f, __uint_as_float(x[q * 4 + e]));   // + the hi * W_lo part
+                            float f = v[q * 4 + e];
                             if (p.bias) f = __fadd_rn(f, b4[e]);
                             if (p.a) f = __fadd_rn(__fmul_rn(a4[e], f), c4[e]);
                             if (p.relu) f = relu_ref(f);
-                            v[q * 4 + e] = __float_as_uint(f);
+                            v[q * 4 + e] = f;
                         }
                     }
                 }
-                if (blk == nblk64 - 1 && okw) {   // the accumulator is in registers: the MMA warp may reuse it
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bar_acc_empty[accbuf]);
-                }
+                if (!RUNS && blk == nblk64 - 1 && okw) release_run();
                 if (et == 0 || et == 32) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the previous block's stores have read the boxes
                 asm volatile("bar.sync 1, %0;" ::"n"(FG_EPILOGUE) : "memory");
-                if (epi_abort) { alive = false; break; }
+                if (epi_abort) { alive = false; return; }
                 if (mine) {
 #pragma unroll
                     for (int q = 0; q < 4; q++)
-                        sts128(stile_addr + (hq >> 1) * FG_TILE_BYTES + r * 128 + ((((hq & 1) * 4 + q) ^ (r & 7)) << 4), v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+                        sts128f(stile_addr + (hq >> 1) * FG_TILE_BYTES + r * 128 + ((((hq & 1) * 4 + q) ^ (r & 7)) << 4), v[q * 4], v[q * 4 + 1], v[q * 4 + 2],
+                                v[q * 4 + 3]);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor stores below read what was just written
                 }
                 asm volatile("bar.sync 1, %0;" ::"n"(FG_EPILOGUE) : "memory");
@@ -310,6 +340,34 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
                                  ::"l"(reinterpret_cast<uint64_t>(&out_map)), "r"(n0 + cb + hb * 32), "r"(tile * 128), "r"(stile_addr + hb * FG_TILE_BYTES) : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
+            };
+            if constexpr (RUNS) {
+                float sum[2][16] = {};   // of this thread's channels of either 64-channel block
+                okw = true;
+                for (int run = 0; run < nruns; run++, i++) {
+                    wait_run();
+                    if (!okw) break;
+#pragma unroll
+                    for (int h = 0; h < 4; h++) {   // eight columns at a time: the sums need the registers
+                        const int blk = h >> 1, c = (h & 1) * 8;
+                        if (blk * 64 + hq * 16 >= n_this) continue;
+                        float f[8];
+                        fg_take<8, STACKED>(f, t_mine + (i % FG_ACCS) * ACC_COLS + blk * 64 + c, n_blk);
+#pragma unroll
+                        for (int e = 0; e < 8; e++) sum[blk][c + e] = __fadd_rn(sum[blk][c + e], f[e]);
+                    }
+                    release_run();
+                }
+                write(sum[0], 0);
+                if (nblk64 > 1 && alive) write(sum[1], 1);
+            } else {
+                wait_run();
+                for (int blk = 0; blk < nblk64 && alive; blk++) {
+                    float v[16];
+                    if (okw && n_this - blk * 64 > hq * 16) fg_take<16, STACKED>(v, t_mine + (i % FG_ACCS) * ACC_COLS + blk * 64, n_blk);
+                    write(v, blk);
+                }
+                i++;
             }
         }
     }

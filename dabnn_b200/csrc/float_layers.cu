@@ -709,10 +709,15 @@ static bool fconv_is_pointwise(int kh, int kw, int pad_h, int pad_w, int stride_
 
 // Shapes of the TMA-fed GEMM kernel: 16-byte channel rows, and windows within the im2col descriptor's fields (corner
 // offsets of a byte, tap offsets below 256, strides up to 8).  Thin inputs (below 16 channels would leave three quarters
-// of every 32-float row empty) stay with the kernels that stage input rows.
+// of every 32-float row empty) stay with the kernels that stage input rows.  Channel counts that are no multiple of 16 have
+// the mma.sync kernel otherwise, whose rounded split is the closer one at short K (distance to float64 at K = 36: 2.9e-7,
+// here 5.8e-7; at 100 0.76 and 0.92e-6; at 216 1.45 and 1.37e-6); a pointwise one of whole channel groups was always here.
 static bool fconv_gemm_takes(int cin, int cout, int kh, int kw, int pad_h, int pad_w, int stride_h, int stride_w, int dil_h, int dil_w) {
     if (cin % 4 || cout % 4 || cin < 16) return false;
-    if (fconv_is_pointwise(kh, kw, pad_h, pad_w, stride_h, stride_w)) return true;
+    const bool pointwise = fconv_is_pointwise(kh, kw, pad_h, pad_w, stride_h, stride_w);
+    if (pointwise && cin % FG_CHUNK == 0) return true;
+    if (cout % 16 && kh * kw * cin < 192) return false;
+    if (pointwise) return true;
     const int far_h = pad_h - (kh - 1) * dil_h, far_w = pad_w - (kw - 1) * dil_w;
     return stride_h <= 8 && stride_w <= 8 && pad_h <= 128 && pad_w <= 128 && far_h >= -128 && far_w >= -128 && far_h <= 127 && far_w <= 127 &&
            (kh - 1) * dil_h < 256 && (kw - 1) * dil_w < 256;
@@ -749,13 +754,12 @@ int fconv_impl(const float* in, const float* weight, const float* bias, const fl
             int optin = 0;
             cudaFuncAttributes fa;
             DABNN_CUDA_OK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-            DABNN_CUDA_OK(cudaFuncGetAttributes(&fa, fconv_gemm_kernel<true>));
+            DABNN_CUDA_OK(cudaFuncGetAttributes(&fa, fconv_gemm_kernel<true, true>));
             gemm_stages = FG_MAX_STAGES;
             while (gemm_stages >= 2 && fg_smem_bytes(gemm_stages) > optin - (int)fa.sharedSizeBytes) gemm_stages--;
-            if (gemm_stages >= 2) {
-                DABNN_CUDA_OK(cudaFuncSetAttribute(fconv_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, fg_smem_bytes(gemm_stages)));
-                DABNN_CUDA_OK(cudaFuncSetAttribute(fconv_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fg_smem_bytes(gemm_stages)));
-            }
+            if (gemm_stages >= 2)
+                for (auto kern : {fconv_gemm_kernel<false, false>, fconv_gemm_kernel<true, false>, fconv_gemm_kernel<true, true>})
+                    DABNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fg_smem_bytes(gemm_stages)));
             gemm_device = dev;
         }
         const int Mpx = n * oh * ow, tiles_m = (Mpx + 127) / 128;
@@ -776,9 +780,10 @@ int fconv_impl(const float* in, const float* weight, const float* bias, const fl
             make_f32_tensor_map(&o_map, out, 2, odims, ostr, box) &&
             (!prm.wgt_rem || make_f32_tensor_map(&wr_map, const_cast<float*>(prm.wgt_rem), 3, wdims, wstr, wbox))) {
             const int items = tiles_m * ((cout + n_blk - 1) / n_blk);
-            const bool stacked = !pointwise && kh * kw * ((cin + FG_CHUNK - 1) / FG_CHUNK) * FG_CHUNK <= FG_STACKED_K;
-            launch_overlapped(stacked ? fconv_gemm_kernel<true> : fconv_gemm_kernel<false>, std::min(items, sm_count()), FG_THREADS,
-                              fg_smem_bytes(gemm_stages), stream, prm, Mpx, gemm_stages, n_blk, (int)!pointwise, a_map, w_map, wr_map, o_map);
+            const int nruns = fg_runs(kh * kw, cin);
+            auto kern = !fg_stacked(pointwise, cin) ? fconv_gemm_kernel<false, false> : nruns > 1 ? fconv_gemm_kernel<true, true> : fconv_gemm_kernel<true, false>;
+            launch_overlapped(kern, std::min(items, sm_count()), FG_THREADS, fg_smem_bytes(gemm_stages), stream, prm, Mpx, gemm_stages, n_blk,
+                              (int)!pointwise, nruns, a_map, w_map, wr_map, o_map);
             return check_launch("fconv_gemm_kernel");
         }
     }

@@ -579,6 +579,36 @@ def test_fconv_im2col_gemm(ops, port, n, h, w, cin, cout, ks, stride, pad, dil, 
     assert ops.engine_status() == 0
 
 
+@pytest.mark.parametrize("h,cin,cout,ks,slices,each", [
+    # stacked form, slices of eight channels in a run: one run, many, windows whose taps end inside a slice (two runs at least)
+    (14, 240, 64, 1, 30, 2), (14, 500, 64, 1, 63, 2), (14, 268, 20, 1, 34, 2), (14, 1024, 64, 1, 128, 2), (14, 16, 64, 3, 18, 2), (14, 20, 64, 3, 15, 2),
+    (14, 28, 64, 3, 20, 2), (14, 60, 64, 2, 16, 2), (14, 20, 64, 5, 39, 2), (14, 128, 64, 3, 144, 2), (14, 132, 64, 3, 51, 2), (14, 256, 64, 3, 144, 2),
+    (14, 512, 64, 3, 144, 2), (14, 512, 64, 5, 144, 2), (7, 512, 64, 7, 144, 2), (1, 25088, 64, 1, 144, 2),
+    (14, 64, 64, 1, 8, 3), (14, 512, 64, 1, 64, 3),                                    # three instructions a slice
+    (14, 20, 20, 1, 0, 0), (14, 36, 20, 1, 0, 0), (14, 100, 20, 1, 0, 0), (14, 16, 20, 2, 0, 0),   # short K and channels in fours: mma.sync
+])
+def test_fconv_distance_to_float64(ops, h, cin, cout, ks, slices, each):
+    """fp32 grade at every K: 2-norm distance to the float64 result.  The accumulators truncate: an instruction that adds to
+    one loses 2^-24 of its binade on average, 0.72 * 2^-24 of its value, which over a run is half the end value on average:
+    2.2e-8, times 1.15.  On top comes the split (3.5e-7 without lo * lo).  The mma.sync kernel: 8e-9 per k and 1.2e-7."""
+    g = torch.Generator(device="cuda").manual_seed(cin * ks)
+    n = 300 if h == 1 else 16 if h == ks else 4
+    x = torch.randn((n, h, h, cin), device="cuda", generator=g)
+    w = torch.randn((cout, ks, ks, cin), device="cuda", generator=g) * (2.0 / (cin * ks * ks)) ** 0.5
+    bias = 0.01 * torch.randn(cout, device="cuda", generator=g)
+    pad = 0 if h == ks else ks // 2
+    got = ops.fconv(x, w, bias, pad, pad, 1, 1).double()
+    xp = torch.nn.functional.pad(x.double(), (0, 0, pad, pad, pad, pad))
+    exact = bias.double() + torch.zeros_like(got)
+    for ky in range(ks):
+        for kx in range(ks):
+            exact += xp[:, ky:ky + got.shape[1], kx:kx + got.shape[2]] @ w[:, ky, kx].double().T
+    limit = 3.5e-7 + 2.5e-8 * slices * each if slices else 1.2e-7 + 8e-9 * ks * ks * cin
+    distance = ((got - exact).norm() / exact.norm()).item()
+    assert distance < limit < 1e-5, (distance, limit)
+    assert ops.engine_status() == 0
+
+
 @pytest.mark.parametrize("cin,cout,ks", [(64, 64, 3), (128, 32, 3), (64, 128, 1), (256, 64, 3)])
 def test_batchnorm_fold_identity(ops, port, cin, cout, ks):
     """The converter's BatchNorm fold for a binary convolution (reference tools/onnx2bnn/OnnxConverter.cpp:583-639:
