@@ -214,6 +214,11 @@ static int check_conv_args(const void* in, const void* weight, size_t weight_wor
     return DABNN_OK;
 }
 
+bool bconv_reads_expanded_weights(int cout, int kwords) {
+    const EpilogueParams ep{nullptr, cout, 0, nullptr, nullptr, nullptr, cout, nullptr, cout / 64, nullptr};
+    return tc5_eligible(ep, cout) && !tmem_takes(ep, cout, kwords);
+}
+
 size_t bconv_expanded_weight_bytes(int cout, int kwords) { return tc5_expanded_bytes(cout, kwords); }
 
 int bconv_expand_weights(const uint64_t* weight, size_t weight_words, int cout, int kwords, unsigned char* dst,

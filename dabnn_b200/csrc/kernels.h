@@ -28,8 +28,9 @@ bool make_u8_tensor_map(CUtensorMap_st* map, const unsigned char* base, int rank
                         const unsigned long long* strides_bytes, const unsigned* box);
 
 // Weights of a binary convolution expanded once to the TCGEN05 engine's stage layout (bytes {0,1}, 8x the packed
-// size): size of the buffer, and the kernel that fills it.  bconv_block_impl takes the buffer as w_expanded.
-// (Read by the kernel for K of more than 255 words; the others expand their filters as they go.)
+// size): whether a block reads them (only the kernel for K of more than 255 words does, the others expand their filters as
+// they go), size of the buffer, and the kernel that fills it.  bconv_block_impl takes the buffer as w_expanded.
+bool bconv_reads_expanded_weights(int cout, int kwords);
 size_t bconv_expanded_weight_bytes(int cout, int kwords);
 int bconv_expand_weights(const uint64_t* weight, size_t weight_words, int cout, int kwords, unsigned char* dst,
                          cudaStream_t stream);

@@ -753,12 +753,17 @@ int NetImpl::build() {
         arena_bytes_extra = 2 * sb;
     }
     if (engine == DABNN_ENGINE_AUTO || engine == DABNN_ENGINE_TCGEN05) {
-        // the weights never change: expand them to the tensor-core engine's byte layout once, not once per pixel tile
+        // the weights never change: where a kernel reads them as bytes, expand them to its layout once, not once per pixel tile
+        auto kwords_of = [&](const Op& o) { return o.kh * o.kw * (blobs[o.in].c / 64); };
+        // (the layer plan, optimize = false, keeps them for every block: its footprint is the yardstick of the fused plan's)
+        auto reads_bytes = [&](const Op& o) {
+            return o.kind == OpKind::BConvBlock && (o.u8 || !optimize || bconv_reads_expanded_weights(blobs[o.out].c, kwords_of(o)));
+        };
         std::vector<size_t> offs;
         for (const Op& o : plan) {
-            if (o.kind != OpKind::BConvBlock) continue;
+            if (!reads_bytes(o)) continue;
             offs.push_back(expanded_bytes);
-            const int kwords = o.kh * o.kw * (blobs[o.in].c / 64);
+            const int kwords = kwords_of(o);
             expanded_bytes += ((o.u8 ? bconv_u8_weight_bytes(blobs[o.out].c, kwords) : bconv_expanded_weight_bytes(blobs[o.out].c, kwords)) + 255) / 256 * 256;
         }
         if (expanded_bytes) {
@@ -768,9 +773,9 @@ int NetImpl::build() {
             }
             size_t k = 0;
             for (Op& o : plan) {
-                if (o.kind != OpKind::BConvBlock) continue;
+                if (!reads_bytes(o)) continue;
                 unsigned char* dst = expanded + offs[k++];
-                const int kwords = o.kh * o.kw * (blobs[o.in].c / 64);
+                const int kwords = kwords_of(o);
                 const int rc = o.u8 ? bconv_u8_expand_weights(static_cast<const uint64_t*>(o.w->dev), o.w->count, blobs[o.out].c, kwords, dst, stream)
                                     : bconv_expand_weights(static_cast<const uint64_t*>(o.w->dev), o.w->count, blobs[o.out].c, kwords, dst, stream);
                 if (rc) return rc;
