@@ -46,7 +46,8 @@ def test_pack_random(ops, port, shape):
 def test_pack_alignments_and_tails(ops, port, size, offset):
     rng = np.random.default_rng(size + offset)
     x = rng.normal(0, 1, size).astype(np.float32)
-    x[rng.random(size) < 0.02] = rng.choice(np.array([0.0, -0.0, np.nan, np.inf, -np.inf, 1e-45], np.float32), 1)
+    odd = rng.random(size) < 0.1
+    x[odd] = rng.choice(np.array([0.0, -0.0, np.nan, np.inf, -np.inf, 1e-45, -1e-45], np.float32), odd.sum())   # one of them at each place
     buf = torch.zeros(size + 16, device="cuda")
     buf[offset:offset + size] = dev_f32(x)
     assert same_bits(host_bits(ops.pack_mat(buf[offset:offset + size].view(1, 1, 1, size))).ravel(), port.pack_64(x).ravel())
@@ -305,13 +306,15 @@ def test_bconv_block_fused_equals_layer_sequence(ops, port, engine, H, cin, cout
 
 
 # n, h, w, words of channels, cout, k, pad, stride: every channel block (128 ... 16 and the kernel for longer K), stages and pixel tiles
-# that end early, odd and even words per tap, channels that end inside a 32-channel item
+# that end early, odd and even words per tap, channels that end inside a 32-channel item; last line: K of more than 255 words, whose
+# operands are both expanded into shared memory
 @pytest.mark.parametrize("n,h,w,cw,cout,k,pad,stride", [
     (1, 1, 1, 1, 16, 1, 0, 1), (1, 127, 1, 4, 128, 1, 0, 1), (1, 43, 3, 5, 144, 1, 0, 1), (150, 16, 8, 8, 64, 1, 0, 1),
     (150, 16, 8, 1, 128, 1, 0, 1), (601, 8, 8, 2, 128, 3, 1, 1), (3, 11, 13, 3, 48, 3, 1, 2), (2, 14, 14, 4, 192, 3, 1, 1),
     (1, 7, 7, 8, 512, 3, 1, 1), (150, 8, 8, 4, 256, 3, 1, 1), (1, 9, 9, 5, 80, 5, 2, 1), (2, 9, 7, 8, 32, 5, 2, 2),
     (1, 5, 5, 9, 16, 5, 2, 1), (64, 14, 14, 8, 512, 3, 1, 1),
-    (106, 14, 14, 8, 512, 3, 1, 1), (160, 12, 12, 3, 80, 5, 2, 1), (4, 6, 6, 12, 64, 5, 2, 1)])
+    (106, 14, 14, 8, 512, 3, 1, 1), (160, 12, 12, 3, 80, 5, 2, 1), (4, 6, 6, 12, 64, 5, 2, 1),
+    (1, 43, 3, 256, 16, 1, 0, 1), (3, 9, 7, 29, 144, 3, 1, 2), (90, 15, 15, 29, 64, 3, 1, 1), (2, 8, 8, 33, 192, 3, 0, 1)])
 def test_bconv_tensor_memory_kernels(ops, port, n, h, w, cw, cout, k, pad, stride):
     rng = np.random.default_rng(h * 100 + cout)
     x, wt = rand_bits(rng, (n, h, w, cw)), rand_bits(rng, cout * k * k * cw)
@@ -485,16 +488,22 @@ def test_float_layers_random(ops, port, shape):
 
 @pytest.mark.parametrize("h,cin,cout,ks,stride,pad,bias", [(32, 3, 64, 7, 2, 3, False), (8, 64, 128, 1, 1, 0, False),
                                                            (1, 512, 1000, 1, 1, 0, True), (9, 5, 7, 3, 1, 1, True),
-                                                           # tensor-memory path: more tiles than SMs, ragged channel blocks,
-                                                           # padded K of 152 / 144 / 256, a partial last pixel tile
+                                                           # the window-reading kernel; the TMA-fed GEMM with ragged channel
+                                                           # blocks, a partial last pixel tile, taps that end inside a slice
                                                            (224, 3, 64, 7, 2, 3, True), (14, 256, 48, 1, 1, 0, True),
                                                            (20, 16, 144, 3, 1, 1, False), (13, 28, 16, 3, 2, 1, True),
                                                            # staged rows: two segments per output row, with 16-byte copies at
                                                            # a non-zero alignment shift and with 4-byte copies
                                                            (136, 3, 16, 3, 1, 1, True), (150, 3, 16, 3, 1, 1, False),
                                                            (132, 4, 32, 5, 1, 2, True),
-                                                           # K = 256: 32-channel weight blocks
-                                                           (7, 256, 96, 1, 1, 0, True)])
+                                                           (7, 256, 96, 1, 1, 0, True),
+                                                           # pixels gathered into tensor-core stages (channels not in fours, or
+                                                           # too few for a GEMM stage): padded K of 16 / 168 / 248, ragged
+                                                           # channel blocks, more tiles than SMs
+                                                           (14, 12, 96, 1, 1, 0, True), (20, 18, 144, 3, 1, 1, False),
+                                                           (13, 27, 16, 3, 2, 1, True), (110, 10, 48, 1, 1, 0, False),
+                                                           # the same, padded K = 256: 32-channel weight blocks
+                                                           (14, 250, 48, 1, 1, 0, True), (7, 254, 96, 1, 1, 0, True)])
 def test_fconv_vs_oracle(ops, port, h, cin, cout, ks, stride, pad, bias):
     rng = np.random.default_rng(h + cin)
     x = rng.normal(0, 1, (2, h, h, cin)).astype(np.float32)
@@ -538,10 +547,10 @@ def test_last_engine_names_the_kernel_that_ran(ops, port):
 
 
 @pytest.mark.parametrize("h,cin,cout,ks,stride,pad,dil", [(16, 5, 7, 3, 1, 2, 2), (20, 16, 32, 3, 1, 2, 2), (23, 3, 16, 3, 2, 2, 2),
-                                                         (12, 64, 64, 1, 1, 0, 2)])
+                                                         (12, 64, 64, 1, 1, 0, 2), (20, 18, 32, 3, 1, 2, 2)])
 def test_fconv_dilation(ops, port, h, cin, cout, ks, stride, pad, dil):
     """Dilated windows (the reference's tests/fconv_test.cpp runs dilation 2) on every route: the mma.sync kernel
-    (Cout % 16 != 0), staged rows, and a 1x1 kernel for which dilation must change nothing."""
+    (Cout % 16 != 0), the TMA-fed GEMM, staged rows (18 channels), and a 1x1 kernel for which dilation must change nothing."""
     rng = np.random.default_rng(h * cin)
     x = rng.normal(0, 1, (2, h, h, cin)).astype(np.float32)
     w = rng.normal(0, np.sqrt(2.0 / (cin * ks * ks)), (cout, ks, ks, cin)).astype(np.float32)
@@ -788,9 +797,9 @@ def test_bconv_u8_block_with_average_pooled_output(ops, port, n, H, cin, cout):
 
 @pytest.mark.parametrize("n,H,cin,cout", [(9, 56, 64, 64), (33, 14, 256, 256), (150, 7, 512, 512)])
 def test_block_kernels_and_their_tunings_agree(ops, n, H, cin, cout):
-    """The two kernels a 3x3 stride-1 block can run on (one TMA box per tap / the tile's halo loaded once), every
-    staging-tile setting of the halo kernel, and launches with and without programmatic overlap give the same bits
-    (the reference has one result per layer: dabnn/layers/BinConv.cpp:144 + Affine.cpp:10 + Add.cpp:7)."""
+    """The two kernels a 3x3 stride-1 block can run on (one TMA box per tap / the tile's halo loaded once) and launches with
+    and without programmatic overlap give the same bits, and the hook ignores its upper bits (the reference has one result
+    per layer: dabnn/layers/BinConv.cpp:144 + Affine.cpp:10 + Add.cpp:7)."""
     from dabnn_b200 import capi
     lib = capi.load()
     rng = np.random.default_rng(n + H)
@@ -803,7 +812,7 @@ def test_block_kernels_and_their_tunings_agree(ops, n, H, cin, cout):
     try:
         lib.dabnn_debug_set_halo(0)
         base = run()
-        for mode in (1, 1 | (2 << 4), 1 | (3 << 4), 1 | ((8 | 3) << 4), 1 | ((8 | 5) << 4)):
+        for mode in (1, 1 | ((8 | 5) << 4)):
             lib.dabnn_debug_set_halo(mode)
             got = run()
             assert ops.engine_status() == 0
