@@ -13,7 +13,7 @@
 // Both operands use the same bit -> K-slot permutation (expand32), which a contraction is blind to.
 //
 // What bounds it: the producers' instruction issue at long K, the epilogue (and HBM: the fp32 output and shortcut) at short K.
-// Against the kernel of bcontract_tc5.cuh, us a launch: block of 256 x 28x28x128 -> 128 3x3 with shortcut 78.5 -> 53.6 (206 MB,
+// Against the kernel of bcontract_tc5.cuh, us a launch: block of 256 x 28x28x128 -> 128 3x3 with shortcut 78.5 -> 53.6 (212 MB,
 // 32 us at the copy rate), 256 x 56x56x64 -> 64 179 -> 98, 256 x 14x14x256 -> 256 72 -> 49; 256 x 14x14x256 -> 512 1x1 49 -> 27;
 // 802816 x 64 x 576 GEMM 150 -> 87; 49 x 512 x 4608 25 -> 10.5.  Left shifts instead of right ones in the expansion: 14x14x256
 // 54 -> 49, 7x7x512 at 32 channels 85 -> 75; groups of producers in turn instead of half a stage each: 72 -> 54.

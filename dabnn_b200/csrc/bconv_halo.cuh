@@ -318,34 +318,32 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
         bool alive = true;
         while (alive && tile < p.ntiles) {
             const int ptile = tile, pchunk = chunk;
-            {
-                // the item after this one, for the shortcut's prefetch
-                int k2 = k, chunk2 = chunk + EPI_GROUPS;
-                while (chunk2 >= nchunk) { chunk2 -= nchunk; k2++; }
-                const int tile2 = tile_of(k2);
-                long long base2 = 0;
-                int nvalid2 = 0;
-                const bool more = tile2 < p.ntiles;
-                if (more) tile_span(tile2, base2, nvalid2);
-                const int accbuf = k % U8_ACCS, cl = chunk * 32 + e.q * 8;
-                    alive = __all_sync(0xffffffffu, mbar_wait<64>(&bar_acc_full[accbuf], (k / U8_ACCS) & 1, abort_flag));
-                if (!alive) {
-                    atomicCAS(&g_u8_status, 0, 24);
-                    s_abort = 1;
-                    epi_abort[group] = 1;
-                } else {
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    e.take(tmem_base + ((uint32_t)r0 << 16) + accbuf * acc_cols + chunk * 32);
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bar_acc_empty[accbuf]);   // this warp's share of the accumulator has been read
-                    if (p.shortcut)
-                        e.finish<true, POOL>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), p.shortcut + element(base2, chunk2), more ? limit_of(nvalid2, chunk2) : 0u);
-                    else
-                        e.finish<false, POOL>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), nullptr, 0u);
-                }
-                k = k2; chunk = chunk2; tile = tile2; base = base2; nvalid = nvalid2;
+            // the item after this one, for the shortcut's prefetch
+            int k2 = k, chunk2 = chunk + EPI_GROUPS;
+            while (chunk2 >= nchunk) { chunk2 -= nchunk; k2++; }
+            const int tile2 = tile_of(k2);
+            long long base2 = 0;
+            int nvalid2 = 0;
+            const bool more = tile2 < p.ntiles;
+            if (more) tile_span(tile2, base2, nvalid2);
+            const int accbuf = k % U8_ACCS, cl = chunk * 32 + e.q * 8;
+            alive = mbar_wait_warp<64>(&bar_acc_full[accbuf], (k / U8_ACCS) & 1, abort_flag);
+            if (!alive) {
+                atomicCAS(&g_u8_status, 0, 24);
+                s_abort = 1;
+                epi_abort[group] = 1;
+            } else {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                e.take(tmem_base + ((uint32_t)r0 << 16) + accbuf * acc_cols + chunk * 32);
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_acc_empty[accbuf]);   // this warp's share of the accumulator has been read
+                if (p.shortcut)
+                    e.finish<true, POOL>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), p.shortcut + element(base2, chunk2), more ? limit_of(nvalid2, chunk2) : 0u);
+                else
+                    e.finish<false, POOL>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), nullptr, 0u);
             }
+            k = k2; chunk = chunk2; tile = tile2; base = base2; nvalid = nvalid2;
             if (POOL) {
                 // 2x2 average pooling of the item
                 group_sync();

@@ -375,9 +375,9 @@ __global__ void __launch_bounds__(U8_THREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar_acc_empty[accbuf]);   // this warp's share of the accumulator has been read
             if (p.shortcut)
-                        e.finish<true, false>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), p.shortcut + element(base2, chunk2), more ? limit_of(nvalid2, chunk2) : 0u);
-                    else
-                        e.finish<false, false>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), nullptr, 0u);
+                e.finish<true, false>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), p.shortcut + element(base2, chunk2), more ? limit_of(nvalid2, chunk2) : 0u);
+            else
+                e.finish<false, false>(o, ch, cl < TC5_MAX_N ? cl : 0, element(base, chunk), limit_of(nvalid, chunk), nullptr, 0u);
             k = k2; chunk = chunk2; tile = tile2; base = base2; nvalid = nvalid2;
         }
     }

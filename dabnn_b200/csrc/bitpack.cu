@@ -33,8 +33,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const float4* __restrict__ in
 // The same for inputs on a 32-byte boundary, 4 KB per warp and step: lane l loads floats 8 l .. 8 l + 7 of each of four 1 KB
 // runs (32-byte loads, all four in flight), which gives one byte per run; two exchanges transpose the 4 x 4 bytes of every four
 // lanes, after which each lane holds a whole 32-bit word and the warp stores 128 contiguous bytes.
-// HBM bounds it (a 64th of what is read is written): 802816 x 576
-// floats in 287 us, 6.6 TB/s of 6.5 copied (16-byte loads with a shuffle per nibble: 330 us).  One wave of the five blocks that
+// HBM bounds it (a 32nd of what is read is written): 802816 x 576 floats in 287 us, 6.6 TB/s of 6.5 copied (16-byte loads with a shuffle per nibble: 330 us).  One wave of the five blocks that
 // fit an SM (48 registers); with a second, partial wave it takes 311 - 316 us.
 __global__ void __launch_bounds__(256) pack_wide_kernel(const float* __restrict__ in, uint32_t* __restrict__ out, const size_t n8) {
     grid_launch_dependents();

@@ -4,8 +4,8 @@
 // K runs over (window tap, 32-channel group).  A stage's pixel tile - 128 consecutive output pixels, 32 floats each - is
 // one TMA load: for 1x1 / stride 1 a box of the [pixels][Cin] matrix, otherwise an im2col-mode load, in which the copy
 // engine itself walks the window positions of 128 output pixels (row and image ends, stride, dilation, zero fill for
-// padding), so a tile has no waste at row ends and every Cin % 4 == 0 window costs the same as a 1x1.  Channels beyond
-// Cin read as zeros in both operands.
+// padding), so a tile has no waste at row ends.  Channels beyond Cin in a tap's last group read as zeros in both operands:
+// they are loaded and split like the others, and only the 8-channel slices that hold channels are multiplied.
 //
 // The tensor core truncates its fp32 operands to tf32, so the raw fp32 tile that a load drops into shared memory
 // (128 rows x 32 floats, 128-byte-swizzled: exactly the K-major layout the MMA reads) IS the head x_hi of the split
@@ -13,11 +13,11 @@
 // layout (same offsets, so the swizzle never has to be undone), for the pixel tile and for the weight tile alike.  The
 // weight remainders follow the weights directly, so per 8-float slice the MMA warp issues hi * [W_hi; W_lo] as one
 // instruction of twice the width - the pixel operand is read once for both - and lo * W_hi, into two halves of a TMEM
-// accumulator that the epilogue adds.
+// accumulator that the epilogue adds (pointwise convolutions of short K: three instructions, fg_stacked).
 //
 // What bounds it: the shared-memory pipe.  Per 128 x 128 x 32 stage the MMAs read 80 KB, the converters move 64 KB and
 // the loads write 32 KB - about 1400 cycles at 128 B per cycle - for 864 cycles of tensor math.  A 3x3 convolution of 64
-// images of 28x28x128 to 128 channels takes 81 us here (182 TFLOP/s of fp32 products, of 340 at the tf32 issue peak); on
+// images of 28x28x128 to 128 channels takes 72 us here (205 TFLOP/s of fp32 products, of 340 at the tf32 issue peak); on
 // the mma.sync kernel, whose threads gather the windows, it took 364 us.
 //
 // One persistent CTA per SM walks (pixel tile, channel block) pairs, channel blocks innermost so that a pixel tile
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1)
     unsigned char* stile = stage0 + stages * FG_STAGE_BYTES;
     const volatile int* abort_flag = &s_abort;
     const int cgroups = (p.cin + FG_CHUNK - 1) / FG_CHUNK, taps = p.kh * p.kw, nchunks = taps * cgroups;
-    // n_blk: channels per work item (32, 64 or 128: small when there are few pixel tiles, so that every SM gets work)
+    // n_blk: channels per work item (a multiple of 32 up to 128: small when there are few pixel tiles, so that every SM gets work)
     const int tiles_m = (M + 127) / 128, nblocks = (p.cout + n_blk - 1) / n_blk;
     const uint32_t w_bytes = (uint32_t)n_blk * 128u;   // a weight tile of a stage
     const int nitems = tiles_m * nblocks;

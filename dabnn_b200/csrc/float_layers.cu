@@ -367,7 +367,7 @@ struct FconvParams {
     const float *in, *wgt, *bias, *a, *b;
     float* out;
     int relu, n, h, w, cin, cout, kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, oh, ow;
-    const float* wgt_rem;   // or null: w - trunc_tf32(w) for every weight, computed once by fconv_split_weights (1x1 GEMM kernel)
+    const float* wgt_rem;   // or null: w - trunc_tf32(w) for every weight, computed once by fconv_split_weights (fconv_gemm.cuh)
 };
 
 __global__ void __launch_bounds__(FNT, 2) fconv_kernel(const FconvParams p) {

@@ -76,7 +76,7 @@ int fconv_impl(const float* in, const float* weight, const float* bias, const fl
                int relu, float* out, int n, int h, int w, int cin, int cout, int kh, int kw, int pad_h,
                int pad_w, int stride_h, int stride_w, int dil_h, int dil_w, cudaStream_t stream, const float* weight_rem = nullptr);
 // weight_rem (optional, 16-byte aligned): the remainders w - trunc_tf32(w) of constant weights, computed once by
-// fconv_split_weights; the 1x1 GEMM kernel then loads them by TMA instead of recomputing them for every tile.
+// fconv_split_weights; the GEMM kernel (fconv_gemm.cuh) then loads them by TMA instead of recomputing them for every tile.
 // fconv_uses_weight_remainders tells for which convolutions they are read.
 int fconv_split_weights(const float* weight, float* rem, size_t count, cudaStream_t stream);
 bool fconv_uses_weight_remainders(int cin, int cout, int kh, int kw, int pad_h, int pad_w, int stride_h, int stride_w);

@@ -785,7 +785,7 @@ int NetImpl::build() {
         }
     }
     if (optimize) {
-        // 1x1 float convolutions run as a TMA-fed GEMM whose tensor core wants x = head + remainder of both operands: the
+        // Most float convolutions run as a TMA-fed GEMM whose tensor core wants x = head + remainder of both operands: the
         // weights' remainders are constants, computed here once instead of once per pixel tile
         std::vector<size_t> offs;
         for (const Op& o : plan) {

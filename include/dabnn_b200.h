@@ -209,7 +209,7 @@ int dabnn_fconv(const float* in, const float* weight, const float* bias, float* 
  * padding 1):  y = conv(in, weight) (+ bias);  if (a) y = a[c]*y + b[c];  if (relu) y = max(y, 0);  out = maxpool3x3s2p1(y).
  * y itself is never written.  out fp32 [n][ph][pw][cout] with ph = (oh - 1) / 2 + 1; out_u8 (optional) = its signs as
  * {0,1} bytes.  The result is bit-identical to dabnn_fconv + dabnn_affine + dabnn_relu + dabnn_maxpool.  Shapes taken:
- * cin <= 4, horizontal stride 2, no dilation, kw <= 8, output rows of 64 .. 128 pixels, cout % 16 == 0
+ * cin <= 3, horizontal stride 2, no dilation, kw <= 8, output rows of 64 .. 128 pixels, cout % 16 == 0
  * (dabnn_fconv_maxpool_supported tells); anything else returns DABNN_ERR_SHAPE. */
 int dabnn_fconv_maxpool_supported(int n, int h, int w, int cin, int cout, int kh, int kw, int pad_h, int pad_w, int stride_h,
                                   int stride_w);
