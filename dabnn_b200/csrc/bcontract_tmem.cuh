@@ -49,7 +49,6 @@ __device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint
 // One 64-bit word of the warp's 32 rows -> 16 tensor-memory columns, K slots as expand32 orders them.  A set bit becomes the byte
 // 128: left shifts are multiplications and leave the logic pipe, which the masks alone keep busy.  The accumulator is scaled
 // back, exactly, in the epilogue.
-constexpr float TM_SCALE = 1.f / 128.f;
 constexpr int TM_MAX_WORDS = (1 << 21) / 128 / 64 - 1;   // |accumulator| stays below 2^21 (EpiWarp::finish)
 __device__ __forceinline__ void tmem_st_word(uint32_t t_addr, uint64_t word) {
     const uint32_t M = 0x80808080u, l = (uint32_t)word, h = (uint32_t)(word >> 32);
@@ -319,7 +318,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
         }
     } else {
         // =========================== epilogue ===========================
-        if (tid - PW * 32 < TC5_MAX_N) pop[tid - PW * 32] = (float)popw[tid - PW * 32] - EPI_POP_BIAS * TM_SCALE;
+        if (tid - PW * 32 < TC5_MAX_N) pop[tid - PW * 32] = epi_pop_scaled(popw[tid - PW * 32]);
         asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");
         tmem_epilogue<EW>(ep, EpiChannels{pop, chan_a, chan_b}, warp - PW, epi_smem, tmem_base, n0, n_this, M, ntiles_m, acc_cols, naccs, narrow,
                           bar_acc_full, bar_acc_empty, &s_abort);
@@ -544,7 +543,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1)
     } else {
         // =========================== epilogue ===========================
         const int x = tid - (TS_PW + TS_FW) * 32;
-        if (x < TS_NBC) pop[x] = (float)popw[x] - EPI_POP_BIAS * TM_SCALE;
+        if (x < TS_NBC) pop[x] = epi_pop_scaled(popw[x]);
         asm volatile("bar.sync 1, %0;" ::"n"(TS_EW * 32) : "memory");
         tmem_epilogue<TS_EW>(ep, EpiChannels{pop, chan_a, chan_b}, warp - TS_PW - TS_FW, epi_smem, tmem_base, n0, n_this, M, ntiles_m, TS_NBC, TS_TILES,
                              narrow, bar_acc_full, bar_acc_empty, &s_abort);

@@ -91,11 +91,16 @@ struct EpiOut {
     int narrow;                   // the shortcut or `out` starts on a 16-byte boundary only
 };
 
-// Per-channel constants as the epilogue reads them: popcount of the weight row less 1.5 * 2^23 (see finish), affine.
+// Per-channel constants as the epilogue reads them: popcount of the weight row as epi_pop or epi_pop_scaled gives it, affine.
 struct EpiChannels {
     const float *pop, *a, *b;     // shared memory
 };
-constexpr float EPI_POP_BIAS = 12582912.f;
+constexpr float EPI_POP_BIAS = 12582912.f;   // 1.5 * 2^23
+// An integer of less than 23 bits (a count is one) added to the bits of 2^23 is 2^23 + that integer as a float: the popcount
+// is kept with those bits added, as an integer.  Accumulators of 128 a bit: an integer of less than 22 bits and a sign added to
+// the bits of 1.5 * 2^23 is 1.5 * 2^23 + that integer; the popcount is kept less the bias, scaled alike.
+__device__ __forceinline__ float epi_pop(int pop) { return __uint_as_float((uint32_t)pop + 0x4B000000u); }
+__device__ __forceinline__ float epi_pop_scaled(int pop) { return (float)pop - EPI_POP_BIAS / 128.f; }
 
 // One warp's side of the epilogue.
 struct EpiWarp {
@@ -160,10 +165,9 @@ struct EpiWarp {
             float y[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) {
-                // an integer of less than 22 bits added to the bits of 1.5 * 2^23 is 1.5 * 2^23 + that integer as a float, and
-                // the sum with popcount - 1.5 * 2^23 is exact (SCALED: accumulators of 128 a bit, the bias in pop scaled alike)
-                const float f = __uint_as_float(t[i] + 0x4B400000u);
-                y[i] = SCALED ? __fmaf_rn(f, 1.f / 128.f, pop[i]) : __fadd_rn(f, pop[i]);
+                // the count, exactly (see epi_pop)
+                y[i] = SCALED ? __fmaf_rn(__uint_as_float(t[i] + 0x4B400000u), 1.f / 128.f, pop[i])
+                              : __fsub_rn(__uint_as_float(t[i] + __float_as_uint(pop[i])), 8388608.f);
                 y[i] = __fadd_rn(__fmul_rn(a[i], y[i]), b[i]);
                 if (SC) y[i] = __fadd_rn(sc[s][i], y[i]);
             }

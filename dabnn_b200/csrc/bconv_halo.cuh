@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(HL_THREADS, 1)
     if (p.imgs == 2 && tid < p.hslots * 4)   // the zero pixel behind the second image's halo (never written again)
         sts128(smem_u32(halo0) + (tid >> 2) * p.halo_stride + (p.img_pitch + (p.rows + 2) * p.P) * 64 + (tid & 3) * 16, 0u, 0u, 0u, 0u);
     if (tid < TC5_MAX_N) {
-        pop[tid] = (tid < n_this ? (float)__ldg(reinterpret_cast<const int*>(p.w_img + u8_weight_image_bytes(p.N, nboxes)) + n0 + tid) : 0.f) - EPI_POP_BIAS;
+        pop[tid] = epi_pop(tid < n_this ? __ldg(reinterpret_cast<const int*>(p.w_img + u8_weight_image_bytes(p.N, nboxes)) + n0 + tid) : 0);
         const bool have = p.a && tid < n_this;
         chan_a[tid] = have ? __ldg(p.a + n0 + tid) : 1.f;
         chan_b[tid] = have ? __ldg(p.b + n0 + tid) : 0.f;

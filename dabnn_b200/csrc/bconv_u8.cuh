@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(U8_THREADS, 1)
         s_abort = 0;
     }
     if (tid < TC5_MAX_N) {
-        pop[tid] = (tid < n_this ? (float)__ldg(reinterpret_cast<const int*>(p.w_img + u8_weight_image_bytes(p.N, p.nboxes)) + n0 + tid) : 0.f) - EPI_POP_BIAS;
+        pop[tid] = epi_pop(tid < n_this ? __ldg(reinterpret_cast<const int*>(p.w_img + u8_weight_image_bytes(p.N, p.nboxes)) + n0 + tid) : 0);
         const bool have = p.a && tid < n_this;
         chan_a[tid] = have ? __ldg(p.a + n0 + tid) : 1.f;
         chan_b[tid] = have ? __ldg(p.b + n0 + tid) : 0.f;

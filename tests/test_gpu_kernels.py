@@ -795,6 +795,21 @@ def test_bconv_u8_block_with_average_pooled_output(ops, port, n, H, cin, cout):
     assert not ops.bconv_u8_block_pooled_supported(n, H, H, cin, cout, 3, 3, 1, 1, 2, 2)       # stride 2
 
 
+@pytest.mark.parametrize("h,w,words,k", [(1, 1, 65537, 1), (7, 14, 7283, 3)])   # the per-tap kernel and the halo kernel
+def test_bconv_u8_block_counts_beyond_22_bits(ops, h, w, words, k):
+    """Counts are exact up to 23 bits: K just above 2^22, every activation set, filters that are all zeros (every bit counts),
+    all ones (only padded taps count) and random, against the packed-bit popcount engine."""
+    cin, cout = 64 * words, 16
+    g = torch.Generator(device="cuda").manual_seed(words)
+    wt = torch.randint(-2**63, 2**63 - 1, (cout, k * k * words), device="cuda", dtype=torch.int64, generator=g)
+    wt[0], wt[1] = 0, -1
+    x8 = torch.ones((1, h, w, cin), device="cuda", dtype=torch.uint8)
+    got = ops.bconv_u8_block(x8, ops.bconv_u8_expand_weights(wt.flatten(), cout, k * k * words), cout, k, k, k // 2, k // 2, 1, 1)[0]
+    exp = ops.bconv(torch.full((1, h, w, words), -1, device="cuda", dtype=torch.int64), wt.flatten(), cout, k, k, k // 2, k // 2, 1, 1, "popc")
+    assert exp.max().item() == k * k * cin > 2**22
+    assert torch.equal(got, exp) and ops.engine_status() == 0
+
+
 @pytest.mark.parametrize("n,H,cin,cout", [(9, 56, 64, 64), (33, 14, 256, 256), (150, 7, 512, 512)])
 def test_block_kernels_and_their_tunings_agree(ops, n, H, cin, cout):
     """The two kernels a 3x3 stride-1 block can run on (one TMA box per tap / the tile's halo loaded once) and launches with
